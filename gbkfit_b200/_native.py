@@ -95,6 +95,7 @@ _SIGS = {
     'gbkb200_ctx_set_stream': [c_void_p, c_void_p],
     'gbkb200_ctx_set_sync': [c_void_p, c_int],
     'gbkb200_ctx_set_mcdisk': [c_void_p, ctypes.c_ulonglong, c_int],
+    'gbkb200_ctx_set_fft': [c_void_p, c_int],
     'gbkb200_ctx_reserve_scratch': [c_void_p, ctypes.c_size_t],
     'gbkb200_mcdisk_scratch_bytes': [c_int, c_int, c_int, c_int],
     'gbkb200_ctx_synchronize': [c_void_p],
@@ -170,6 +171,11 @@ class Context:
 
     def set_mcdisk(self, seed, mode=0):
         check(_lib.gbkb200_ctx_set_mcdisk(self.handle, int(seed), int(mode)), 'set_mcdisk')
+
+    def set_fft(self, mode):
+        """0: two-factor transforms where the line lengths have them; 1: the
+        mixed-radix passes for every length (include/gbkb200.h)."""
+        check(_lib.gbkb200_ctx_set_fft(self.handle, int(mode)), 'set_fft')
 
     def reserve_scratch(self, nbytes):
         check(_lib.gbkb200_ctx_reserve_scratch(self.handle, int(nbytes)), 'reserve_scratch')

@@ -78,6 +78,14 @@ extern "C" int gbkb200_ctx_set_mcdisk(gbkb200_ctx* ctx, unsigned long long seed,
     return GBKB200_OK;
 }
 
+extern "C" int gbkb200_ctx_set_fft(gbkb200_ctx* ctx, int mode)
+{
+    if (!ctx || mode < 0 || mode > 1) return GBKB200_ERR_INVALID_ARG;
+    if (ctx->fft_mode == mode) return GBKB200_OK;
+    ctx->fft_mode = mode;
+    return gbk_fft_state_destroy(ctx);      // its plans hold the other kernels
+}
+
 extern "C" int gbkb200_ctx_reserve_scratch(gbkb200_ctx* ctx, size_t bytes)
 {
     if (!ctx) return GBKB200_ERR_INVALID_ARG;

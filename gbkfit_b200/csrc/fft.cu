@@ -10,7 +10,8 @@
 //
 // Kernels (all passes in shared memory, self-sorting mixed-radix Stockham with
 // radices 8/4/2/3/5/7 and a generic odd-prime butterfly up to 61; twiddles
-// are computed on the host in double precision):
+// are computed on the host in double precision), for the line lengths that
+// the two-factor register transforms of gbk_lines.cuh do not cover:
 //   x_r2c   rows of the real cube, as nx/2-point complex FFTs plus the
 //           even/odd split (nx even) or full complex FFTs (nx odd);
 //   lines   tiles of 16 adjacent columns along y or z, one 128-byte
@@ -18,7 +19,7 @@
 //   conv_z  the z pass fused with the pointwise multiply and the inverse z
 //           pass: a column is read once and written once;
 //   x_c2r   the inverse of x_r2c.
-#include "gbk_fft.cuh"
+#include "gbk_lines.cuh"
 
 #include <array>
 #include <cmath>
@@ -34,7 +35,8 @@ namespace gbk {
 // post: exp(-2 pi i k / nx) for k in [0, nx/2].  Shared memory:
 // 2 * L * M complex + M twiddles + (nx/2 + 1) post twiddles.
 __global__ void __launch_bounds__(FFT_THREADS) x_r2c_kernel(const float* in, float2* out, int rows,
-                                                            int nx, AxisDev ax, const float2* post)
+                                                            int nx, int pitch, AxisDev ax,
+                                                            const float2* post)
 {
     extern __shared__ float2 sm[];
     const int M = ax.n;
@@ -81,13 +83,14 @@ __global__ void __launch_bounds__(FFT_THREADS) x_r2c_kernel(const float* in, flo
         } else {
             X = z[l * M + k];
         }
-        out[row * hx + k] = X;
+        out[row * pitch + k] = X;
     }
 }
 
 // Inverse of x_r2c (unnormalised, like FFTW's c2r).
 __global__ void __launch_bounds__(FFT_THREADS) x_c2r_kernel(const float2* in, float* out, int rows,
-                                                            int nx, AxisDev ax, const float2* post)
+                                                            int nx, int pitch, AxisDev ax,
+                                                            const float2* post)
 {
     extern __shared__ float2 sm[];
     const int M = ax.n;
@@ -110,7 +113,7 @@ __global__ void __launch_bounds__(FFT_THREADS) x_c2r_kernel(const float2* in, fl
             [&](int e) {
                 const int l = fdiv(e, ax.mn), k = e - l * M;
                 const long long row = row0 + l;
-                return row < rows ? in[row * hx + k] : make_float2(0.f, 0.f);
+                return row < rows ? in[row * pitch + k] : make_float2(0.f, 0.f);
             },
             [&](int e, float2 v) { b0[e] = v; });
         staged_copy<8>(
@@ -118,7 +121,7 @@ __global__ void __launch_bounds__(FFT_THREADS) x_c2r_kernel(const float2* in, fl
             [&](int e) {
                 const int l = fdiv(e, ax.mn), k = e - l * M;
                 const long long row = row0 + l;
-                return row < rows ? in[row * hx + M - k] : make_float2(0.f, 0.f);
+                return row < rows ? in[row * pitch + M - k] : make_float2(0.f, 0.f);
             },
             [&](int e, float2 v) { b1[e] = v; });
         __syncthreads();
@@ -138,7 +141,7 @@ __global__ void __launch_bounds__(FFT_THREADS) x_c2r_kernel(const float2* in, fl
                 const int l = fdiv(e, ax.mn), k = e - l * M;
                 const long long row = row0 + l;
                 if (row >= rows) return make_float2(0.f, 0.f);
-                const float2* r = in + row * hx;
+                const float2* r = in + row * pitch;
                 return k < hx ? r[k] : conjf2(r[nx - k]);
             },
             [&](int e, float2 v) { b0[e] = v; });
@@ -230,13 +233,17 @@ struct Axis {
 
 struct Plan {
     int nx = 0, ny = 0, nz = 0, hx = 0;
+    int pitch = 0;            // row pitch of the plan's own spectra (128-byte rows)
     Axis ax, ay, az;
+    FastRows fx;              // two-factor kernels, where the lengths have them
+    FastLines fy, fz;
     float2* post = nullptr;   // exp(-2 pi i k / nx), k in [0, nx/2]
 };
 
 using Size3 = std::array<int, 3>;
 
 struct FftState {
+    int mode = 0;                                               // gbkb200_ctx_set_fft
     std::map<Size3, Plan> plans;
     std::map<std::pair<Size3, const void*>, float2*> spectra;   // cached data2 spectra
     std::map<Size3, float2*> work;                              // data1 spectra
@@ -292,6 +299,7 @@ static int get_plan(FftState* st, const Size3& s, Plan** out)
     if (it != st->plans.end()) { *out = &it->second; return GBKB200_OK; }
     Plan p;
     p.nx = s[0]; p.ny = s[1]; p.nz = s[2]; p.hx = p.nx / 2 + 1;
+    p.pitch = (p.hx + FAST_LT - 1) / FAST_LT * FAST_LT;
     if (p.nx < 1 || p.ny < 1 || p.nz < 1) return GBKB200_ERR_INVALID_ARG;
     const int M = (p.nx % 2 == 0 && p.nx > 1) ? p.nx / 2 : p.nx;
     if (rows_smem(M, p.nx) > SMEM_LIMIT || lines_smem(p.ny, lines_tile(p.ny)) > SMEM_LIMIT ||
@@ -301,6 +309,11 @@ static int get_plan(FftState* st, const Size3& s, Plan** out)
     if ((rc = make_axis(p.ax, M))) return rc;
     if ((rc = make_axis(p.ay, p.ny))) return rc;
     if ((rc = make_axis(p.az, p.nz))) return rc;
+    if (st->mode == 0) {
+        if (p.nx % 2 == 0) p.fx = fast_rows(M);
+        p.fy = fast_lines(p.ny);
+        p.fz = fast_lines(p.nz);
+    }
     std::vector<float2> post(p.hx);
     for (int k = 0; k < p.hx; ++k) {
         double ang = -2.0 * M_PI * (double)k / (double)p.nx;
@@ -318,97 +331,129 @@ static int set_smem(const void* fn, size_t bytes)
     return gbk_raise_smem_limit(fn, bytes);
 }
 
-// x-pass launch helpers
-static int launch_r2c(const Plan& p, const float* in, float2* out, cudaStream_t st)
+// x-pass launch helpers; pitch: row pitch of the spectrum
+static int launch_r2c(const Plan& p, const float* in, float2* out, int pitch, cudaStream_t st)
 {
     if ((reinterpret_cast<uintptr_t>(in) & 7) || (reinterpret_cast<uintptr_t>(out) & 7))
         return GBKB200_ERR_INVALID_ARG;   // rows are read as float2 pairs
     const int rows = p.ny * p.nz;
     const int M = p.ax.dev.n;
-    const int L = std::max(1, std::min(16, 8192 / M));
-    size_t smem = rows_smem(M, p.nx);
-    int rc = set_smem((const void*)x_r2c_kernel, smem);
-    if (rc) return rc;
-    x_r2c_kernel<<<(rows + L - 1) / L, FFT_THREADS, smem, st>>>(in, out, rows, p.nx, p.ax.dev, p.post);
+    int rc;
+    if (p.fx.fwd) {
+        if ((rc = set_smem((const void*)p.fx.fwd, p.fx.smem))) return rc;
+        p.fx.fwd<<<(rows + FAST_LT - 1) / FAST_LT, p.fx.threads, p.fx.smem, st>>>(
+            in, out, rows, pitch, p.ax.tw, p.post);
+    } else {
+        const int L = std::max(1, std::min(16, 8192 / M));
+        size_t smem = rows_smem(M, p.nx);
+        if ((rc = set_smem((const void*)x_r2c_kernel, smem))) return rc;
+        x_r2c_kernel<<<(rows + L - 1) / L, FFT_THREADS, smem, st>>>(in, out, rows, p.nx, pitch,
+                                                                    p.ax.dev, p.post);
+    }
     GBK_CUDA_TRY(cudaGetLastError());
     return GBKB200_OK;
 }
 
-static int launch_c2r(const Plan& p, const float2* in, float* out, cudaStream_t st)
+static int launch_c2r(const Plan& p, const float2* in, float* out, int pitch, cudaStream_t st)
 {
     if ((reinterpret_cast<uintptr_t>(in) & 7) || (reinterpret_cast<uintptr_t>(out) & 7))
         return GBKB200_ERR_INVALID_ARG;
     const int rows = p.ny * p.nz;
     const int M = p.ax.dev.n;
-    const int L = std::max(1, std::min(16, 8192 / M));
-    size_t smem = rows_smem(M, p.nx);
-    int rc = set_smem((const void*)x_c2r_kernel, smem);
-    if (rc) return rc;
-    x_c2r_kernel<<<(rows + L - 1) / L, FFT_THREADS, smem, st>>>(in, out, rows, p.nx, p.ax.dev, p.post);
+    int rc;
+    if (p.fx.inv) {
+        if ((rc = set_smem((const void*)p.fx.inv, p.fx.smem))) return rc;
+        p.fx.inv<<<(rows + FAST_LT - 1) / FAST_LT, p.fx.threads, p.fx.smem, st>>>(
+            in, out, rows, pitch, p.ax.tw, p.post);
+    } else {
+        const int L = std::max(1, std::min(16, 8192 / M));
+        size_t smem = rows_smem(M, p.nx);
+        if ((rc = set_smem((const void*)x_c2r_kernel, smem))) return rc;
+        x_c2r_kernel<<<(rows + L - 1) / L, FFT_THREADS, smem, st>>>(in, out, rows, p.nx, pitch,
+                                                                    p.ax.dev, p.post);
+    }
     GBK_CUDA_TRY(cudaGetLastError());
     return GBKB200_OK;
 }
 
 // y or z pass over the complex cube (mode 0: single transform; mode 1: conv)
-static int launch_lines(const Plan& p, float2* data, int axis, int inv, int mode,
+static int launch_lines(const Plan& p, float2* data, int pitch, int axis, int inv, int mode,
                         const float2* spec, float scale, cudaStream_t st)
 {
     const Axis& a = axis == 1 ? p.ay : p.az;
     if (a.dev.n == 1 && mode == 0) return GBKB200_OK;
-    const int lt = lines_tile(a.dev.n);
-    const int tiles = (p.hx + lt - 1) / lt;
     long long so, sk;
-    int outer;
-    if (axis == 1) { outer = p.nz; so = (long long)p.ny * p.hx; sk = p.hx; }
-    else { outer = p.ny; so = p.hx; sk = (long long)p.ny * p.hx; }
-    size_t smem = lines_smem(a.dev.n, lt);
-    auto kern = lt == 16 ? lines_kernel<16> : lines_kernel<8>;
-    int rc = set_smem((const void*)kern, smem);
-    if (rc) return rc;
-    kern<<<outer * tiles, FFT_THREADS, smem, st>>>(data, p.hx, so, sk, a.dev, inv, mode, spec,
-                                                   scale);
+    int outer, rc;
+    if (axis == 1) { outer = p.nz; so = (long long)p.ny * pitch; sk = pitch; }
+    else { outer = p.ny; so = pitch; sk = (long long)p.ny * pitch; }
+    const FastLines& f = axis == 1 ? p.fy : p.fz;
+    const FastLinesFn fn = f.fn[mode == 1 ? 2 : inv ? 1 : 0];
+    if (fn) {
+        const int tiles = (p.hx + FAST_LT - 1) / FAST_LT;
+        if ((rc = set_smem((const void*)fn, f.smem))) return rc;
+        fn<<<outer * tiles, f.threads, f.smem, st>>>(data, p.hx, tiles, so, sk, a.tw, spec, scale);
+    } else {
+        const int lt = lines_tile(a.dev.n);
+        const int tiles = (p.hx + lt - 1) / lt;
+        size_t smem = lines_smem(a.dev.n, lt);
+        auto kern = lt == 16 ? lines_kernel<16> : lines_kernel<8>;
+        if ((rc = set_smem((const void*)kern, smem))) return rc;
+        kern<<<outer * tiles, FFT_THREADS, smem, st>>>(data, p.hx, so, sk, a.dev, inv, mode, spec,
+                                                       scale);
+    }
     GBK_CUDA_TRY(cudaGetLastError());
     return GBKB200_OK;
 }
 
 // x and y passes of the forward transform (the z pass is fused with the
 // spectrum multiply in convolve_tail)
-static int forward_xy(const Plan& p, const float* r, float2* c, cudaStream_t st)
+static int forward_xy(const Plan& p, const float* r, float2* c, int pitch, cudaStream_t st)
 {
     int rc;
-    if ((rc = launch_r2c(p, r, c, st))) return rc;
-    return launch_lines(p, c, 1, 0, 0, nullptr, 1.f, st);
+    if ((rc = launch_r2c(p, r, c, pitch, st))) return rc;
+    return launch_lines(p, c, pitch, 1, 0, 0, nullptr, 1.f, st);
 }
 
-static int forward(const Plan& p, const float* r, float2* c, cudaStream_t st)
+static int forward(const Plan& p, const float* r, float2* c, int pitch, cudaStream_t st)
 {
     int rc;
-    if ((rc = forward_xy(p, r, c, st))) return rc;
-    return launch_lines(p, c, 2, 0, 0, nullptr, 1.f, st);
+    if ((rc = forward_xy(p, r, c, pitch, st))) return rc;
+    return launch_lines(p, c, pitch, 2, 0, 0, nullptr, 1.f, st);
 }
 
 // c holds the x/y-transformed cube: forward z, multiply by spec * scale,
 // inverse z (one fused pass), then inverse y and c2r into r
-static int convolve_tail(const Plan& p, float2* c, const float2* spec, float* r, cudaStream_t st)
+static int convolve_tail(const Plan& p, float2* c, const float2* spec, float* r, int pitch,
+                         cudaStream_t st)
 {
     int rc;
     // fft.hpp:185-197: nfactor = T{1} / (n0 * n1 * n2) in T
     const float scale = 1.0f / (float)(p.nx * p.ny * p.nz);
     if (p.nz > 1) {
-        if ((rc = launch_lines(p, c, 2, 0, 1, spec, scale, st))) return rc;
+        if ((rc = launch_lines(p, c, pitch, 2, 0, 1, spec, scale, st))) return rc;
     } else {
-        long long n = (long long)p.nz * p.ny * p.hx;
+        long long n = (long long)p.nz * p.ny * pitch;
         cmul_scale_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 32), 256, 0, st>>>(
             c, spec, n, scale);
         GBK_CUDA_TRY(cudaGetLastError());
     }
-    if ((rc = launch_lines(p, c, 1, 1, 0, nullptr, 1.f, st))) return rc;
-    return launch_c2r(p, c, r, st);
+    if ((rc = launch_lines(p, c, pitch, 1, 1, 0, nullptr, 1.f, st))) return rc;
+    return launch_c2r(p, c, r, pitch, st);
+}
+
+// a spectrum at the plan's own (padded) pitch
+static size_t spectrum_bytes(const Plan& p)
+{
+    return (size_t)p.nz * p.ny * p.pitch * sizeof(float2);
 }
 
 static FftState* state(gbkb200_ctx* ctx)
 {
-    if (!ctx->fft_state) ctx->fft_state = new FftState();
+    if (!ctx->fft_state) {
+        FftState* st = new FftState();
+        st->mode = ctx->fft_mode;
+        ctx->fft_state = st;
+    }
     return static_cast<FftState*>(ctx->fft_state);
 }
 
@@ -457,7 +502,7 @@ extern "C" int gbkb200_fft_r2c_f32(gbkb200_ctx* ctx, const int size[3], const fl
     if ((rc = get_size(size, s))) return rc;
     Plan* p;
     if ((rc = get_plan(state(ctx), s, &p))) return rc;
-    if ((rc = forward(*p, data_r, static_cast<float2*>(data_c), ctx->stream))) return rc;
+    if ((rc = forward(*p, data_r, static_cast<float2*>(data_c), p->hx, ctx->stream))) return rc;
     return gbk_finish(ctx);
 }
 
@@ -474,11 +519,11 @@ extern "C" int gbkb200_fft_c2r_f32(gbkb200_ctx* ctx, const int size[3], const vo
     // work on a copy so that data_c is preserved
     float2*& w = st->work[s];
     size_t bytes = (size_t)p->nz * p->ny * p->hx * sizeof(float2);
-    if (!w) GBK_CUDA_TRY(cudaMalloc(&w, bytes));
+    if (!w) GBK_CUDA_TRY(cudaMalloc(&w, spectrum_bytes(*p)));
     GBK_CUDA_TRY(cudaMemcpyAsync(w, data_c, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    if ((rc = launch_lines(*p, w, 2, 1, 0, nullptr, 1.f, ctx->stream))) return rc;
-    if ((rc = launch_lines(*p, w, 1, 1, 0, nullptr, 1.f, ctx->stream))) return rc;
-    if ((rc = launch_c2r(*p, w, data_r, ctx->stream))) return rc;
+    if ((rc = launch_lines(*p, w, p->hx, 2, 1, 0, nullptr, 1.f, ctx->stream))) return rc;
+    if ((rc = launch_lines(*p, w, p->hx, 1, 1, 0, nullptr, 1.f, ctx->stream))) return rc;
+    if ((rc = launch_c2r(*p, w, data_r, p->hx, ctx->stream))) return rc;
     return gbk_finish(ctx);
 }
 
@@ -494,8 +539,9 @@ extern "C" int gbkb200_fft_convolve_f32(gbkb200_ctx* ctx, const int size[3], flo
     // data1_c is work space: the reference multiplies in place and runs
     // FFTW's multi-dimensional c2r on it, which destroys it (fft.hpp:199-207)
     float2* c = static_cast<float2*>(data1_c);
-    if ((rc = forward_xy(*p, data1_r, c, ctx->stream))) return rc;
-    if ((rc = convolve_tail(*p, c, static_cast<const float2*>(data2_c), data1_r, ctx->stream)))
+    if ((rc = forward_xy(*p, data1_r, c, p->hx, ctx->stream))) return rc;
+    if ((rc = convolve_tail(*p, c, static_cast<const float2*>(data2_c), data1_r, p->hx,
+                            ctx->stream)))
         return rc;
     return gbk_finish(ctx);
 }
@@ -510,20 +556,20 @@ extern "C" int gbkb200_fft_convolve_cached_f32(gbkb200_ctx* ctx, const int size[
     FftState* st = state(ctx);
     Plan* p;
     if ((rc = get_plan(st, s, &p))) return rc;
-    size_t bytes = (size_t)p->nz * p->ny * p->hx * sizeof(float2);
+    const size_t bytes = spectrum_bytes(*p);
     auto key = std::make_pair(s, (const void*)data2_r);
     auto it = st->spectra.find(key);
     float2* spec;
     if (it == st->spectra.end()) {
         if (cudaMalloc(&spec, bytes) != cudaSuccess) return GBKB200_ERR_OOM;
         st->spectra[key] = spec;
-        if ((rc = forward(*p, data2_r, spec, ctx->stream))) return rc;
+        if ((rc = forward(*p, data2_r, spec, p->pitch, ctx->stream))) return rc;
     } else {
         spec = it->second;
     }
     float2*& w = st->work[s];
     if (!w && cudaMalloc(&w, bytes) != cudaSuccess) return GBKB200_ERR_OOM;
-    if ((rc = forward_xy(*p, data1_r, w, ctx->stream))) return rc;
-    if ((rc = convolve_tail(*p, w, spec, data1_r, ctx->stream))) return rc;
+    if ((rc = forward_xy(*p, data1_r, w, p->pitch, ctx->stream))) return rc;
+    if ((rc = convolve_tail(*p, w, spec, data1_r, p->pitch, ctx->stream))) return rc;
     return gbk_finish(ctx);
 }

@@ -72,6 +72,7 @@ struct gbkb200_ctx {
     int sync = 1;
     unsigned long long seed = 42;
     int mc_mode = 0;
+    int fft_mode = 0;             // 1: mixed-radix passes only (gbkb200_ctx_set_fft)
     int* d_status = nullptr;      // device status word (GBK_STATUS_* bits)
     int* h_status = nullptr;      // pinned mirror
     void* fft_state = nullptr;    // FFT plan / spectrum caches (fft.cu)

@@ -551,6 +551,10 @@ class DModelMMaps:
         dc = self._dcube
         if self._driver is not driver or self._gmodel is not gmodel:
             dc.prepare(driver, gmodel.has_weights())
+            # the second moment weighs the cube's rounding by the squared
+            # velocity: faint spaxels move by ~5e-5 with other transforms, so
+            # the maps keep the ones they came from so far
+            dc._backend_fft._ctx.set_fft(1)
             self._backend = driver.backends().dmodel(dc.dtype())
             n = len(self._orders)
             ny, nx = self.size()[1], self.size()[0]

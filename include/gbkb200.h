@@ -72,6 +72,13 @@ int gbkb200_ctx_set_sync(gbkb200_ctx* ctx, int sync);
  * scube (no scratch).  The assigned maps (wdata, vdata_cmp, ddata_cmp) keep
  * the reference's last-writer-wins race in every mode. */
 int gbkb200_ctx_set_mcdisk(gbkb200_ctx* ctx, unsigned long long seed, int mode);
+/* The transforms of the context's FFT convolutions: 0 (the default) the
+ * two-factor register transforms for the line lengths that have one, 1 the
+ * mixed-radix passes for every length.  They differ in the last bits; the
+ * gradient and the moment maps, which hand out or amplify those, keep the
+ * passes, so that their results stay what they were.
+ * Drops the context's plans and cached spectra. */
+int gbkb200_ctx_set_fft(gbkb200_ctx* ctx, int mode);
 /* grows the context's mcdisk scratch to at least `bytes` now (a later call
  * that needs no more allocates nothing on its stream's path) */
 int gbkb200_ctx_reserve_scratch(gbkb200_ctx* ctx, size_t bytes);
