@@ -53,6 +53,8 @@ _lib.gbkb200_batch_evaluate.restype = c_int
 _lib.gbkb200_batch_info.argtypes = [c_void_p, c_int * 3, ctypes.POINTER(c_int),
                                     ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(c_int)]
 _lib.gbkb200_batch_info.restype = c_int
+_lib.gbkb200_batch_planewise.argtypes = [c_void_p]
+_lib.gbkb200_batch_planewise.restype = c_int
 _lib.gbkb200_batch_destroy.argtypes = [c_void_p]
 _lib.gbkb200_batch_destroy.restype = c_int
 _lib.gbkb200_batch_set_timing.argtypes = [c_void_p, c_int]
@@ -78,6 +80,7 @@ STAGE_KERNELS = {
     'direct': {0: 'ka_lines_lsf', 4: 'kb_psf_residual', 5: 'k6_sum'},
     'fft': {0: 'k1_model_xfft', 1: 'k_lines (y forward)', 2: 'k_lines (z convolution)',
             3: 'k_lines (y inverse)', 4: 'k5_c2r_residual', 5: 'k6_sum'},
+    'planes': {0: 'ka_lines_lsf', 1: 'kp_rows', 2: 'kp_cols', 4: 'kp_resid', 5: 'k6_sum'},
 }
 
 
@@ -505,7 +508,8 @@ class BatchedSMDisk:
         ms = (ctypes.c_double * 6)()
         n = (c_int * 6)()
         check(_lib.gbkb200_batch_timing(self.handle, ms, n), 'batch_timing')
-        names = STAGE_KERNELS[self.conv_mode]
+        planes = _lib.gbkb200_batch_planewise(self.handle)
+        names = STAGE_KERNELS['planes' if planes else self.conv_mode]
         return {names[i]: (ms[i], n[i]) for i in range(6) if n[i]}
 
     def work_counters(self):

@@ -25,8 +25,13 @@
 //   K6  per set, the partials summed in a fixed order in fp64.
 // Sets run in chunks whose intermediates (Wz x Py x hx complex each) stay in
 // the 126 MB L2 between stages.
+//
+// K1-K5 serve windows beyond the plane-wise form's (gbk_planes.cuh) and LSFs
+// longer than the model kernel's FIR; setup_direct and setup_planes say what
+// those take.
 #include "gbk_batched.cuh"
 #include "gbk_fft.cuh"
+#include "gbk_planes.cuh"
 
 #include <climits>
 #include <mutex>
@@ -354,6 +359,15 @@ struct gbkb200_batch {
     float* iw = nullptr;
     void (*kb)(BatchKernelArgs) = nullptr;
     void (*ka)(BatchKernelArgs, int*) = nullptr;
+    // plane-wise FFT convolution (gbk_planes.cuh)
+    int planes = 0;
+    int wave = 0;                     // sets per sub-wave
+    PlaneArgs K{};
+    PlaneRows pr;
+    PlaneCols pc;
+    float2* ptab = nullptr;           // twiddles of both axes, PSF spectrum
+    float2* pconv = nullptr;          // crop rows of the convolved spectra
+    unsigned char* pflags = nullptr;
     // per-stage timing: event pairs recorded around launches while enabled
     int timing = 0;
     int count = 0;                            // work counters on (timing mode 1)
@@ -399,6 +413,18 @@ static void launch_kb(const gbkb200_batch* bt, BatchKernelArgs& P, int cn, cudaS
     } else {
         bt->kb<<<dim3(cn, P.Nz * P.nbands), bt->kb_threads, bt->smemB, st>>>(P);
     }
+}
+
+// the model kernel over cn sets: variants 2-4 a block per (4 rows, chunk),
+// otherwise a warp per item
+static void launch_ka(const gbkb200_batch* bt, const BatchKernelArgs& P, int cn, cudaStream_t st)
+{
+    const bool tiles = bt->ka_variant >= 2;
+    const int items = P.Wy * (bt->ka_variant == 1 ? (P.nch + 1) / 2 : P.nch);
+    const int blocks = tiles ? (P.Wy + 3) / 4 * P.nch
+                             : (items + KA_THREADS / 32 - 1) / (KA_THREADS / 32);
+    const size_t smem = tiles ? (size_t)P.Nz * 16 : 0;
+    bt->ka<<<dim3(blocks, cn), KA_THREADS, smem, st>>>(P, bt->ctx->d_status);
 }
 
 static KaFn ka_fn(int Kz)
@@ -453,6 +479,41 @@ static KbFn kb_fn(int K, int variant)
     return t[variant][(K - KB_KMIN) / 2];
 }
 
+// the node-wise fast path of the spaxel evaluation: exactly one trait of
+// uid 101 for rpt, vpt, dpt and none of the other kinds
+static bool nodewise(const gbkb200_batch_desc* d)
+{
+    bool fast = !d->loose && !d->tilted;
+    for (int k = 0; k < 9 && fast; ++k) {
+        const bool want = k == 0 || k == 2 || k == 4;
+        if (!want) {
+            fast = d->ntraits[k] == 0;
+            continue;
+        }
+        int uid = 0;
+        fast = d->ntraits[k] == 1 && d->uids[k] &&
+               cudaMemcpy(&uid, d->uids[k], sizeof(int), cudaMemcpyDeviceToHost) ==
+                   cudaSuccess &&
+               uid == 101;
+    }
+    return fast;
+}
+
+// Taps below 2^-35 of their factor's largest are dropped from both ends
+// (symmetrically, the centre stays): they change no output by more than
+// ~1e-10 of its peak, below fp32 resolution.  The evaluation window then
+// starts t taps later along each axis and is 2 t shorter, so every kept
+// tap meets the same model voxel as before.
+static int trimmed_taps(const double* a, int n)
+{
+    double m = 0;
+    for (int i = 0; i < n; ++i) m = std::max(m, std::fabs(a[i]));
+    const double thr = std::ldexp(m, -35);
+    int t = 0;
+    while (2 * t + 1 < n && std::fabs(a[t]) < thr && std::fabs(a[n - 1 - t]) < thr) ++t;
+    return t;
+}
+
 // Direct-mode setup: reversed FIR coefficients, plane buffers, the data's
 // summed-area table and shared memory sizes.  Returns
 // GBKB200_ERR_UNSUPPORTED when the direct path does not apply (PSF rank or
@@ -461,21 +522,9 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
 {
     BatchKernelArgs& P = bt->P;
     if (d->psf_rank != 1 || !d->psf_u || !d->psf_v) return GBKB200_ERR_UNSUPPORTED;
-    // Taps below 2^-35 of their factor's largest are dropped from both ends
-    // (symmetrically, the centre stays): they change no output by more than
-    // ~1e-10 of its peak, below fp32 resolution.  The evaluation window then
-    // starts t taps later along each axis and is 2 t shorter, so every kept
-    // tap meets the same model voxel as before.
-    auto trim = [](const double* a, int n) {
-        double m = 0;
-        for (int i = 0; i < n; ++i) m = std::max(m, std::fabs(a[i]));
-        const double thr = std::ldexp(m, -35);
-        int t = 0;
-        while (2 * t + 1 < n && std::fabs(a[t]) < thr && std::fabs(a[n - 1 - t]) < thr) ++t;
-        return t;
-    };
-    const int tx = trim(d->psf_v, d->kernel_size[0]), ty = trim(d->psf_u, d->kernel_size[1]);
-    const int tz = trim(d->lsf, d->kernel_size[2]);
+    const int tx = trimmed_taps(d->psf_v, d->kernel_size[0]);
+    const int ty = trimmed_taps(d->psf_u, d->kernel_size[1]);
+    const int tz = trimmed_taps(d->lsf, d->kernel_size[2]);
     bt->trim[0] = tx; bt->trim[1] = ty; bt->trim[2] = tz;
     P.Kx = d->kernel_size[0] - 2 * tx;
     P.Ky = d->kernel_size[1] - 2 * ty;
@@ -496,24 +545,7 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     const int NW = (P.K + 7 + 3) / 4;
     P.pitch = (P.Wx + 31) / 32 * 32;
     P.nch = (P.Wx + 31) / 32;
-    // the node-wise fast path of the spaxel evaluation: exactly one trait of
-    // uid 101 for rpt, vpt, dpt and none of the other kinds
-    {
-        bool fast = !d->loose && !d->tilted;
-        for (int k = 0; k < 9 && fast; ++k) {
-            const bool want = k == 0 || k == 2 || k == 4;
-            if (!want) {
-                fast = d->ntraits[k] == 0;
-                continue;
-            }
-            int uid = 0;
-            fast = d->ntraits[k] == 1 && d->uids[k] &&
-                   cudaMemcpy(&uid, d->uids[k], sizeof(int), cudaMemcpyDeviceToHost) ==
-                       cudaSuccess &&
-                   uid == 101;
-        }
-        P.nwfast = fast ? 1 : 0;
-    }
+    P.nwfast = nodewise(d) ? 1 : 0;
     int band = d->psf_band > 0 ? std::min(d->psf_band, P.Ny) : P.Ny;
     P.nbands = (P.Ny + band - 1) / band;
     P.band = (P.Ny + P.nbands - 1) / P.nbands;
@@ -604,6 +636,133 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     return GBKB200_OK;
 }
 
+// Set-up of the plane-wise FFT convolution (gbk_planes.cuh): the model kernel
+// with the LSF's FIR, then a 2-D FFT per plane.  Returns
+// GBKB200_ERR_UNSUPPORTED where the LSF is longer than the FIR kernels' or a
+// window than the instantiated transforms.
+static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
+{
+    BatchKernelArgs& P = bt->P;
+    const int tz = trimmed_taps(d->lsf, d->kernel_size[2]);
+    const int Kz = d->kernel_size[2] - 2 * tz;
+    if (Kz > KA_KMAX || P.Wx > KP_MAX_W || P.Wy > KP_MAX_W) return GBKB200_ERR_UNSUPPORTED;
+    bt->pr = plane_rows(P.Wx);
+    bt->pc = plane_cols(P.Wy);
+    if (!bt->pr.rows || !bt->pc.fn) return GBKB200_ERR_UNSUPPORTED;
+    P.Kz = Kz;
+    P.Wz = P.Nz + Kz - 1;
+    P.disk.spec_size = P.Wz;
+    P.disk.spec_zero = d->spec_zero + tz * d->spec_step;
+    P.pitch = (P.Wx + 31) / 32 * 32;
+    P.nch = P.pitch / 32;
+    P.nwfast = nodewise(d) ? 1 : 0;
+    for (int t = 0; t < 33; ++t)
+        P.lsfr[t] = t < Kz ? (float)d->lsf[d->kernel_size[2] - 1 - tz - t] : 0.f;
+    // the model kernel as in the direct mode (the tile forms keep 16 bytes per
+    // plane in shared memory)
+    const int mv = d->model_variant < 0 || d->model_variant > 4 ? 3 : d->model_variant;
+    bt->ka_variant = mv >= 2 && (long long)P.Nz * 16 > 32 * 1024 ? 0 : mv;
+    bt->ka = bt->ka_variant == 1   ? ka2_fn(Kz)
+             : bt->ka_variant >= 2 ? ka_t_fn(Kz, bt->ka_variant - 2)
+                                   : ka_fn(Kz);
+    PlaneArgs& K = bt->K;
+    const int px = bt->pr.n, hx = px / 2 + 1, n = bt->pc.n;
+    K.Nx = P.Nx; K.Ny = P.Ny; K.Nz = P.Nz; K.Wx = P.Wx; K.Wy = P.Wy;
+    K.nch = P.nch; K.pitch = P.pitch;
+    K.hxp = (hx + KP_L - 1) / KP_L * KP_L;
+    K.ngw = (P.Wy + KP_L - 1) / KP_L;
+    // sets per sub-wave: at most 256 MB of spectra.  Keeping them in L2 does
+    // not pay (64 sets of 128 x 128 x 96, spectra of 24 / 48 / 100 / 220 MB per
+    // sub-wave: 1381 / 1107 / 1008 / 972 us; the passes are bound by issue and
+    // small launches leave the chip idle); beyond that only memory grows
+    const size_t per_set = (size_t)P.Nz * K.ngw * KP_L * K.hxp * sizeof(float2);
+    bt->wave = (int)std::max<size_t>(1, std::min<size_t>(bt->chunk, (256u << 20) / per_set));
+    // tables, in 64-bit arithmetic: twiddles of both axes and the
+    // spectrum of the PSF image shifted by its last tap to the origin, so that
+    // the convolution's value at window index i is the crop's at i
+    std::vector<float2> tab((size_t)px + n + (size_t)n * K.hxp, make_float2(0.f, 0.f));
+    auto unit = [](int k, int len) {
+        const double ang = -2.0 * M_PI * (double)k / (double)len;
+        return std::make_pair(std::cos(ang), std::sin(ang));
+    };
+    std::vector<std::pair<double, double>> wx(px), wy(n);
+    for (int k = 0; k < px; ++k) wx[k] = unit(k, px);
+    for (int k = 0; k < n; ++k) wy[k] = unit(k, n);
+    float2* t = tab.data();
+    for (int k = 0; k < px; ++k) *t++ = make_float2((float)wx[k].first, (float)wx[k].second);
+    for (int k = 0; k < n; ++k) *t++ = make_float2((float)wy[k].first, (float)wy[k].second);
+    {
+        const int kx = d->kernel_size[0], ky = d->kernel_size[1];
+        std::vector<double> re((size_t)ky * hx), im((size_t)ky * hx), ar(hx), ai(hx);
+        for (int y = 0; y < ky; ++y)
+            for (int k = 0; k < hx; ++k) {
+                double sr = 0, si = 0;
+                for (int x = 0; x < kx; ++x) {
+                    const auto& w = wx[(int)(((long long)(x - (kx - 1) + px) * k) % px)];
+                    sr += d->psf[y * kx + x] * w.first;
+                    si += d->psf[y * kx + x] * w.second;
+                }
+                re[(size_t)y * hx + k] = sr;
+                im[(size_t)y * hx + k] = si;
+            }
+        const double scale = 1.0 / ((double)px * n);
+        for (int q = 0; q < n; ++q) {
+            std::fill(ar.begin(), ar.end(), 0.0);
+            std::fill(ai.begin(), ai.end(), 0.0);
+            for (int y = 0; y < ky; ++y) {
+                const auto& w = wy[(int)(((long long)(y - (ky - 1) + n) * q) % n)];
+                const double *r = &re[(size_t)y * hx], *i = &im[(size_t)y * hx];
+                for (int k = 0; k < hx; ++k) {
+                    ar[k] += r[k] * w.first - i[k] * w.second;
+                    ai[k] += r[k] * w.second + i[k] * w.first;
+                }
+            }
+            for (int k = 0; k < hx; ++k)
+                t[((size_t)(k / KP_L) * n + q) * KP_L + k % KP_L] =
+                    make_float2((float)(ar[k] * scale), (float)(ai[k] * scale));
+        }
+    }
+    const size_t rows = (size_t)bt->wave * P.Nz * P.Wy;
+    bt->nper = P.Nz * ((P.Ny + KP_L - 1) / KP_L);
+    if (cudaMalloc(&bt->mplanes, rows * P.pitch * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&bt->xrt, rows * P.nch * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&bt->work, bt->wave * per_set) != cudaSuccess ||
+        cudaMalloc(&bt->pconv, (size_t)bt->wave * P.Nz * P.Ny * K.hxp * sizeof(float2)) !=
+            cudaSuccess ||
+        cudaMalloc(&bt->pflags, (size_t)bt->wave * P.Nz * 32) != cudaSuccess ||
+        cudaMalloc(&bt->iw, (size_t)P.Nz * P.Ny * P.Nx * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&bt->ptab, tab.size() * sizeof(float2)) != cudaSuccess ||
+        cudaMalloc(&bt->partials, (size_t)bt->max_sets * bt->nper * sizeof(double)) != cudaSuccess)
+        return GBKB200_ERR_OOM;
+    GBK_CUDA_TRY(cudaMemcpy(bt->ptab, tab.data(), tab.size() * sizeof(float2),
+                            cudaMemcpyHostToDevice));
+    P.mplanes = bt->mplanes;
+    P.xrt = bt->xrt;
+    P.iw = bt->iw;
+    P.partials = bt->partials;
+    k_iw<<<592, 256, 0, bt->ctx->stream>>>(P, bt->iw, (long long)P.Nz * P.Ny * P.Nx);
+    GBK_CUDA_TRY(cudaGetLastError());
+    GBK_CUDA_TRY(cudaStreamSynchronize(bt->ctx->stream));
+    K.mplanes = bt->mplanes;
+    K.xrt = bt->xrt;
+    K.work = bt->work;
+    K.conv = bt->pconv;
+    K.flags = bt->pflags;
+    K.twx = bt->ptab;
+    K.twy = K.twx + px;
+    K.spec = K.twy + n;
+    K.obs = P.obs;
+    K.iw = bt->iw;
+    K.partials = bt->partials;
+    int rc;
+    if ((rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->pr.rows), bt->pr.smem)) ||
+        (rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->pr.resid), bt->pr.smem)) ||
+        (rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->pc.fn), bt->pc.smem)))
+        return rc;
+    bt->planes = 1;
+    return GBKB200_OK;
+}
+
 static bool fft_factor_ok(int n)
 {
     for (int p : {2, 3, 5, 7})
@@ -660,6 +819,9 @@ extern "C" int gbkb200_batch_destroy(gbkb200_batch* bt)
     for (cudaEvent_t e : bt->ev) cudaEventDestroy(e);
     if (bt->done) cudaEventDestroy(bt->done);
     cudaFree(bt->kb_work);
+    cudaFree(bt->ptab);
+    cudaFree(bt->pflags);
+    cudaFree(bt->pconv);
     delete bt;
     return GBKB200_OK;
 }
@@ -745,6 +907,32 @@ extern "C" int gbkb200_batch_create(gbkb200_ctx* ctx, const gbkb200_batch_desc* 
             return rc;
         }
     }
+    // shared memory sizes, set once here so evaluate() can be captured
+    const int M = P.Px / 2;
+    bt->smem1 = (size_t)(2 * P.rows_k1 * M + M + P.hx) * sizeof(float2) +
+                (size_t)P.Wx * (4 * sizeof(float) + 2 * sizeof(int));
+    bt->smem5 = (size_t)(2 * P.rows_k5 * M + M + P.hx) * sizeof(float2);
+    bt->smem_y = (size_t)(2 * BLT * P.Py + P.Py) * sizeof(float2);
+    bt->smem_z = (size_t)(2 * BLT * P.Pz + P.Pz) * sizeof(float2);
+    const size_t lim = 227 * 1024;
+    if (bt->smem1 > lim || bt->smem5 > lim || bt->smem_y > lim || bt->smem_z > lim) {
+        gbkb200_batch_destroy(bt);
+        return GBKB200_ERR_UNSUPPORTED;
+    }
+    {
+        const BatchKernelArgs saved = P;     // its set-up trims the spectral window
+        rc = setup_planes(bt, d);
+        if (rc == GBKB200_OK) {
+            GBK_CUDA_TRY(cudaGetLastError());
+            *out = bt;
+            return GBKB200_OK;
+        }
+        if (rc != GBKB200_ERR_UNSUPPORTED) {
+            gbkb200_batch_destroy(bt);
+            return rc;
+        }
+        P = saved;
+    }
     // post twiddles of the x axis
     {
         std::vector<float2> h(P.hx);
@@ -808,18 +996,6 @@ extern "C" int gbkb200_batch_create(gbkb200_ctx* ctx, const gbkb200_batch_desc* 
     P.lim_work = (long long)bt->chunk * P.Wz * P.Py * P.hx;
     P.lim_part = (long long)bt->max_sets * bt->nper;
     P.lim_obs = (long long)P.Nx * P.Ny * P.Nz;
-    // shared memory sizes, set once here so evaluate() can be captured
-    const int M = P.Px / 2;
-    bt->smem1 = (size_t)(2 * P.rows_k1 * M + M + P.hx) * sizeof(float2) +
-                (size_t)P.Wx * (4 * sizeof(float) + 2 * sizeof(int));
-    bt->smem5 = (size_t)(2 * P.rows_k5 * M + M + P.hx) * sizeof(float2);
-    bt->smem_y = (size_t)(2 * BLT * P.Py + P.Py) * sizeof(float2);
-    bt->smem_z = (size_t)(2 * BLT * P.Pz + P.Pz) * sizeof(float2);
-    const size_t lim = 227 * 1024;
-    if (bt->smem1 > lim || bt->smem5 > lim || bt->smem_y > lim || bt->smem_z > lim) {
-        gbkb200_batch_destroy(bt);
-        return GBKB200_ERR_UNSUPPORTED;
-    }
     if ((rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(k1_model_xfft), bt->smem1)) ||
         (rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(k5_c2r_residual), bt->smem5)) ||
         (rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(k_lines),
@@ -850,6 +1026,12 @@ extern "C" int gbkb200_batch_info(const gbkb200_batch* bt, int fft_size[3], int*
             b += nrows * P.pitch * sizeof(float) + nrows * P.nch * sizeof(int) +
                  (size_t)P.Nz * (P.Ny + 1) * (P.Nx + 1) * sizeof(double) +
                  (size_t)P.Nz * P.Ny * P.Nx * sizeof(float);
+        } else if (bt->planes) {
+            const size_t nrows = (size_t)bt->wave * P.Nz * P.Wy;
+            b += nrows * (P.pitch * sizeof(float) + P.nch * sizeof(int)) +
+                 (size_t)bt->wave * P.Nz * (bt->K.ngw * KP_L + P.Ny) * bt->K.hxp * sizeof(float2) +
+                 (size_t)bt->wave * P.Nz * 32 + (size_t)P.Nz * P.Ny * P.Nx * sizeof(float) +
+                 ((size_t)bt->pr.n + (size_t)bt->pc.n * (1 + bt->K.hxp)) * sizeof(float2);
         } else {
             b += (size_t)bt->chunk * P.Wz * P.Py * P.hx * sizeof(float2) +
                  (size_t)P.Pz * P.Py * P.hx * sizeof(float2) +
@@ -859,6 +1041,8 @@ extern "C" int gbkb200_batch_info(const gbkb200_batch* bt, int fft_size[3], int*
     }
     return GBKB200_OK;
 }
+
+extern "C" int gbkb200_batch_planewise(const gbkb200_batch* bt) { return bt && bt->planes; }
 
 extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float* vsys,
                                       const float* xpos, const float* ypos, const float* posa,
@@ -889,16 +1073,37 @@ extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float*
             const int cn = std::min(bt->chunk, nsets - s0);
             P.set0 = s0;
             stage_mark(bt, 0, true);
-            // variants 2 and 3: a block per (4 rows, chunk); otherwise a warp per item
-            const bool tiles = bt->ka_variant >= 2;
-            const int items = P.Wy * (bt->ka_variant == 1 ? (P.nch + 1) / 2 : P.nch);
-            const int blocks = tiles ? (P.Wy + 3) / 4 * P.nch
-                                     : (items + KA_THREADS / 32 - 1) / (KA_THREADS / 32);
-            const size_t smem = tiles ? (size_t)P.Nz * 16 : 0;
-            bt->ka<<<dim3(blocks, cn), KA_THREADS, smem, st>>>(P, bt->ctx->d_status);
+            launch_ka(bt, P, cn, st);
             stage_mark(bt, 0, false);
             stage_mark(bt, 4, true);
             launch_kb(bt, P, cn, st);
+            stage_mark(bt, 4, false);
+        }
+        stage_mark(bt, 5, true);
+        if (nsets > 0) k6_sum<<<nsets, 256, 0, st>>>(P.partials, bt->nper, 0, chi2);
+        stage_mark(bt, 5, false);
+        GBK_CUDA_TRY(cudaGetLastError());
+        return gbk_finish(bt->ctx);
+    }
+    if (bt->planes) {
+        PlaneArgs K = bt->K;
+        K.model = model;
+        for (int s0 = 0; s0 < nsets; s0 += bt->wave) {
+            const int cn = std::min(bt->wave, nsets - s0);
+            P.set0 = K.set0 = s0;
+            stage_mark(bt, 0, true);
+            launch_ka(bt, P, cn, st);
+            stage_mark(bt, 0, false);
+            stage_mark(bt, 1, true);
+            bt->pr.rows<<<dim3(K.ngw, K.Nz, cn), bt->pr.threads, bt->pr.smem, st>>>(K);
+            stage_mark(bt, 1, false);
+            stage_mark(bt, 2, true);
+            bt->pc.fn<<<dim3(K.hxp / KP_L, K.Nz, cn), bt->pc.threads, bt->pc.smem, st>>>(
+                K, bt->pr.n / 2 + 1);
+            stage_mark(bt, 2, false);
+            stage_mark(bt, 4, true);
+            bt->pr.resid<<<dim3((K.Ny + KP_L - 1) / KP_L, K.Nz, cn), bt->pr.threads, bt->pr.smem,
+                           st>>>(K);
             stage_mark(bt, 4, false);
         }
         stage_mark(bt, 5, true);

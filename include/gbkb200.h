@@ -433,6 +433,9 @@ int gbkb200_batch_take_status(gbkb200_batch* b);
  * 2 = direct) */
 int gbkb200_batch_info(const gbkb200_batch* b, int fft_size[3], int* chunk, size_t* work_bytes,
                        int* conv_mode);
+/* 1 where the FFT mode convolves plane by plane (2-D transforms after the
+ * LSF's FIR), 0 where it transforms the cube (or the mode is direct) */
+int gbkb200_batch_planewise(const gbkb200_batch* b);
 int gbkb200_batch_destroy(gbkb200_batch* b);
 
 /* The batched evaluator's input rows from raw node values, on the device
