@@ -347,10 +347,7 @@ struct gbkb200_batch {
     int nper = 0;
     int direct = 0;
     int trim[3] = {0, 0, 0};          // direct mode: taps trimmed from each end (x, y, z)
-    int ka_variant = 0;               // direct mode: the model kernel (model_variant)
-    int kb_grid = 0;                  // persistent PSF kernel: blocks of a launch (else 0)
-    int kb_threads = KB_THREADS;      // threads of a PSF-kernel block
-    int* kb_work = nullptr;           // persistent PSF kernel: its item counter
+    bool ka_tiles = false;            // the model kernel is the tile form
     cudaEvent_t done = nullptr;       // recorded at the end of an asynchronous submission
     size_t smemB = 0;
     float* mplanes = nullptr;
@@ -400,30 +397,20 @@ static void stage_mark(gbkb200_batch* bt, int stage, bool begin)
     }
 }
 
-// the PSF kernel over cn sets: a block per (set, plane, band), or the
-// persistent variant's resident wave over all of them
-static void launch_kb(const gbkb200_batch* bt, BatchKernelArgs& P, int cn, cudaStream_t st)
+// the PSF kernel over cn sets: a block per (set, plane, band)
+static void launch_kb(const gbkb200_batch* bt, const BatchKernelArgs& P, int cn, cudaStream_t st)
 {
-    if (bt->kb_grid > 0) {
-        P.kb_cn = cn;
-        const long long items = (long long)cn * P.Nz * P.nbands;
-        const int grid = (int)std::min<long long>(items, bt->kb_grid);
-        cudaMemsetAsync(bt->kb_work, 0, sizeof(int), st);
-        bt->kb<<<grid, bt->kb_threads, bt->smemB, st>>>(P);
-    } else {
-        bt->kb<<<dim3(cn, P.Nz * P.nbands), bt->kb_threads, bt->smemB, st>>>(P);
-    }
+    bt->kb<<<dim3(cn, P.Nz * P.nbands), KB_THREADS, bt->smemB, st>>>(P);
 }
 
-// the model kernel over cn sets: variants 2-4 a block per (4 rows, chunk),
-// otherwise a warp per item
+// the model kernel over cn sets: tiles a block per (4 rows, chunk), otherwise
+// a warp per (row, chunk)
 static void launch_ka(const gbkb200_batch* bt, const BatchKernelArgs& P, int cn, cudaStream_t st)
 {
-    const bool tiles = bt->ka_variant >= 2;
-    const int items = P.Wy * (bt->ka_variant == 1 ? (P.nch + 1) / 2 : P.nch);
-    const int blocks = tiles ? (P.Wy + 3) / 4 * P.nch
-                             : (items + KA_THREADS / 32 - 1) / (KA_THREADS / 32);
-    const size_t smem = tiles ? (size_t)P.Nz * 16 : 0;
+    const int blocks = bt->ka_tiles
+                           ? (P.Wy + 3) / 4 * P.nch
+                           : (P.Wy * P.nch + KA_THREADS / 32 - 1) / (KA_THREADS / 32);
+    const size_t smem = bt->ka_tiles ? (size_t)P.Nz * 16 : 0;
     bt->ka<<<dim3(blocks, cn), KA_THREADS, smem, st>>>(P, bt->ctx->d_status);
 }
 
@@ -437,25 +424,32 @@ static KaFn ka_fn(int Kz)
     return t[Kz / 2];
 }
 
-// form 0: ballot masks, 1: transposed masks, 2: transposed masks and the scaled line
-static KaFn ka_t_fn(int Kz, int form)
+static KaFn ka_t_fn(int Kz, bool sl)
 {
-    static KaFn t[3][KA_KMAX / 2 + 1] = {};
+    static KaFn t[2][KA_KMAX / 2 + 1] = {};
     static std::once_flag once;
     std::call_once(once, [] {
-        ka_t_register(t[0], false, false);
-        ka_t_register(t[1], true, false);
-        ka_t_register(t[2], true, true);
+        ka_t_register(t[0], false);
+        ka_t_register(t[1], true);
     });
-    return t[form][Kz / 2];
+    return t[sl][Kz / 2];
 }
 
-static KaFn ka2_fn(int Kz)
+// The model kernel of a model_variant (0-4; 0-3 named forms with identical
+// values): the tile kernel, with the scaled line exponent for 4, or a warp per
+// 32-column chunk where `tiles` is off (the tiles keep 16 bytes per output
+// plane in shared memory).
+static void pick_ka(gbkb200_batch* bt, int variant, bool tiles)
 {
-    static KaFn t[KA_KMAX / 2 + 1] = {};
-    static std::once_flag once;
-    std::call_once(once, [] { ka2_register(t); });
-    return t[Kz / 2];
+    bt->ka_tiles = tiles;
+    bt->ka = tiles ? ka_t_fn(bt->P.Kz, variant == 4) : ka_fn(bt->P.Kz);
+}
+
+// the float4 rows of the residual (BatchKernelArgs::vec)
+static int vector_rows(const BatchKernelArgs& P, const float* model)
+{
+    return P.Nx % 4 == 0 && ((reinterpret_cast<uintptr_t>(P.obs) |
+                              reinterpret_cast<uintptr_t>(model)) & 15) == 0;
 }
 
 static KcFn kc_fn(int Kz)
@@ -466,17 +460,12 @@ static KcFn kc_fn(int Kz)
     return t[Kz / 2];
 }
 
-static KbFn kb_fn(int K, int variant)
+static KbFn kb_fn(int K)
 {
-    static KbFn t[KB_VARIANTS][(KB_KMAX - KB_KMIN) / 2 + 1] = {};
+    static KbFn t[(KB_KMAX - KB_KMIN) / 2 + 1] = {};
     static std::once_flag once;
-    std::call_once(once, [] {
-        kb_register4(t);
-        kb_register5(t + 3);
-        kb_register_pf(t + 6);
-        kb_register_wide(t + 7);
-    });
-    return t[variant][(K - KB_KMIN) / 2];
+    std::call_once(once, [] { kb_register(t); });
+    return t[(K - KB_KMIN) / 2];
 }
 
 // the node-wise fast path of the spaxel evaluation: exactly one trait of
@@ -554,27 +543,16 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     // otherwise 54 KB (four blocks per SM)
     int bpmax = 4 * (2 * ((P.Nx + 7) / 8 - 1) + NW);
     bpmax += ((4 - bpmax % 32) + 32) % 32;
-    // range entries of the band's input rows (the persistent variant 6: two
-    // buffers, each rounded to 4 entries)
-    const bool pf = d->psf_variant == 6;
-    const long long xr_slot = ((long long)(P.band + P.K - 1) * P.nch + 3) & ~3LL;
-    const long long xr_bytes = pf ? 2 * xr_slot * (long long)sizeof(int)
-                                  : (long long)(P.band + P.K - 1) * P.nch * sizeof(int);
+    // range entries of the band's input rows
+    const long long xr_bytes = (long long)(P.band + P.K - 1) * P.nch * sizeof(int);
     const long long need_min = (long long)(P.K + 15) * bpmax;
     const long long need_all = (long long)(P.band + P.K + 7) * bpmax;
-    // PSF kernel variant: 0-2 sized for 4 resident blocks per SM, 3-5 for 5,
-    // epilogue (variant % 3) as in kb_psf_residual, 6 = 0 as a persistent
-    // kernel; shared memory per block: 55 KB for 4 blocks per SM, 43 KB for 5
-    if (d->psf_variant < 0 || d->psf_variant >= KB_VARIANTS) return GBKB200_ERR_INVALID_ARG;
-    const bool wide = d->psf_variant == 7;
-    const int blocks = (d->psf_variant >= 3 && d->psf_variant <= 5) ? 5 : 4;
-    // variant 7: 256-thread blocks, two per SM, 110 KB each
-    const long long budget = wide ? 110LL * 1024 : blocks == 5 ? 43LL * 1024 : 55LL * 1024;
-    bt->kb_threads = wide ? 256 : KB_THREADS;
-    const long long cap = std::max(need_min, std::min(need_all, (budget - xr_bytes) / 4));
+    // psf_variant chose among forms of the PSF kernel that were slower at every
+    // size; its values are accepted and mean the same kernel
+    if (d->psf_variant < 0 || d->psf_variant > 7) return GBKB200_ERR_INVALID_ARG;
+    const long long cap = std::max(need_min, std::min(need_all, (55LL * 1024 - xr_bytes) / 4));
     if (cap * (long long)sizeof(float) + xr_bytes > 227LL * 1024) return GBKB200_ERR_UNSUPPORTED;
     P.cap = (int)cap;
-    P.xr_slot = pf ? (int)xr_slot : 0;
     bt->smemB = (size_t)cap * sizeof(float) + (size_t)xr_bytes;
     std::vector<float> vr(P.K, 0.f), ur(P.K, 0.f), lr(P.Kz);
     for (int s = 0; s < P.Kx; ++s) vr[s] = (float)d->psf_v[d->kernel_size[0] - 1 - tx - s];
@@ -585,7 +563,6 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
         P.vr[i] = i < P.K ? vr[i] : 0.f;
         P.ur[i] = i < P.K ? ur[i] : 0.f;
         P.lsfr[i] = i < P.Kz ? lr[i] : 0.f;
-        P.ur2[i] = make_float2(P.ur[i], P.ur[i]);
     }
     if (cudaMalloc(&bt->mplanes, nrows * P.pitch * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&bt->xrt, nrows * P.nch * sizeof(int)) != cudaSuccess ||
@@ -602,29 +579,14 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     GBK_CUDA_TRY(cudaGetLastError());
     GBK_CUDA_TRY(cudaStreamSynchronize(bt->ctx->stream));
     if (d->model_variant < 0 || d->model_variant > 4) return GBKB200_ERR_INVALID_ARG;
-    // variants 2-4 (4 x 8 tiles) keep a plane's entries of its 4 rows in
-    // shared memory; 3 forms the masks by bit transposes; 4 is 3 with the
-    // scaled line exponent
-    const bool tiles = d->model_variant >= 2;
-    if (tiles && (long long)P.Nz * 16 > 32 * 1024) return GBKB200_ERR_UNSUPPORTED;
-    bt->ka = d->model_variant == 1 ? ka2_fn(P.Kz)
-             : tiles               ? ka_t_fn(P.Kz, d->model_variant - 2)
-                                   : ka_fn(P.Kz);
-    bt->ka_variant = d->model_variant;
-    bt->kb = kb_fn(P.K, d->psf_variant);
+    // variants 2-4 name the tile kernel, which has to fit
+    const bool fits = (long long)P.Nz * 16 <= 32 * 1024;
+    if (d->model_variant >= 2 && !fits) return GBKB200_ERR_UNSUPPORTED;
+    pick_ka(bt, d->model_variant, fits);
+    bt->kb = kb_fn(P.K);
     {
         const int rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->kb), bt->smemB);
         if (rc) return rc;
-    }
-    if (pf) {
-        // one resident wave of blocks
-        int per_sm = 0, nsm = 0;
-        GBK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, reinterpret_cast<const void*>(bt->kb), bt->kb_threads, bt->smemB));
-        GBK_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, bt->ctx->device));
-        bt->kb_grid = std::max(1, per_sm) * std::max(1, nsm);
-        if (cudaMalloc(&bt->kb_work, sizeof(int)) != cudaSuccess) return GBKB200_ERR_OOM;
-        P.kb_work = bt->kb_work;
     }
     bt->nper = P.Nz * P.nbands;
     if (cudaMalloc(&bt->partials, (size_t)bt->max_sets * bt->nper * sizeof(double)) != cudaSuccess)
@@ -658,13 +620,8 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     P.nwfast = nodewise(d) ? 1 : 0;
     for (int t = 0; t < 33; ++t)
         P.lsfr[t] = t < Kz ? (float)d->lsf[d->kernel_size[2] - 1 - tz - t] : 0.f;
-    // the model kernel as in the direct mode (the tile forms keep 16 bytes per
-    // plane in shared memory)
     const int mv = d->model_variant < 0 || d->model_variant > 4 ? 3 : d->model_variant;
-    bt->ka_variant = mv >= 2 && (long long)P.Nz * 16 > 32 * 1024 ? 0 : mv;
-    bt->ka = bt->ka_variant == 1   ? ka2_fn(Kz)
-             : bt->ka_variant >= 2 ? ka_t_fn(Kz, bt->ka_variant - 2)
-                                   : ka_fn(Kz);
+    pick_ka(bt, mv, (long long)P.Nz * 16 <= 32 * 1024);
     PlaneArgs& K = bt->K;
     const int px = bt->pr.n, hx = px / 2 + 1, n = bt->pc.n;
     K.Nx = P.Nx; K.Ny = P.Ny; K.Nz = P.Nz; K.Wx = P.Wx; K.Wy = P.Wy;
@@ -818,7 +775,6 @@ extern "C" int gbkb200_batch_destroy(gbkb200_batch* bt)
     cudaFree(bt->counters);
     for (cudaEvent_t e : bt->ev) cudaEventDestroy(e);
     if (bt->done) cudaEventDestroy(bt->done);
-    cudaFree(bt->kb_work);
     cudaFree(bt->ptab);
     cudaFree(bt->pflags);
     cudaFree(bt->pconv);
@@ -1064,6 +1020,7 @@ extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float*
     }
     P.model = model;
     P.lim_model = model ? (long long)nsets * P.Nz * P.Ny * P.Nx : 0;
+    P.vec = vector_rows(P, model);
     P.counters = bt->count ? bt->counters : nullptr;
     const long long set_stride = (long long)P.Wz * P.Py * P.hx;
     const long long lim_spec = (long long)P.Pz * P.Py * P.hx;
@@ -1088,6 +1045,7 @@ extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float*
     if (bt->planes) {
         PlaneArgs K = bt->K;
         K.model = model;
+        K.vec = vector_rows(P, model);
         for (int s0 = 0; s0 < nsets; s0 += bt->wave) {
             const int cn = std::min(bt->wave, nsets - s0);
             P.set0 = K.set0 = s0;
@@ -1170,6 +1128,7 @@ extern "C" int gbkb200_batch_evaluate_cubes(gbkb200_batch* bt, int nsets, const 
     cudaStream_t st = bt->ctx->stream;
     P.model = model;
     P.lim_model = model ? (long long)nsets * P.Nz * P.Ny * P.Nx : 0;
+    P.vec = vector_rows(P, model);
     P.counters = bt->count ? bt->counters : nullptr;
     const KcFn kc = kc_fn(P.Kz);
     for (int s0 = 0; s0 < nsets; s0 += bt->chunk) {

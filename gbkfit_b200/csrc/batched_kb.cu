@@ -1,57 +1,15 @@
-// Explicit instantiations of the batched PSF kernel sized for 4 resident
-// blocks per SM, every epilogue variant (one translation unit per group, so
-// that the library compiles in parallel).
+// Explicit instantiations of the batched PSF kernel, one per odd FIR length.
 #include "gbk_batched.cuh"
 
 namespace gbk {
 
-void kb_register4(KbFn (*t)[(KB_KMAX - KB_KMIN) / 2 + 1])
+template<int K>
+static void fill(KbFn* t)
 {
-    t[0][0] = kb_psf_residual<5, 4, 0, false, KB_THREADS>;
-    t[0][1] = kb_psf_residual<7, 4, 0, false, KB_THREADS>;
-    t[0][2] = kb_psf_residual<9, 4, 0, false, KB_THREADS>;
-    t[0][3] = kb_psf_residual<11, 4, 0, false, KB_THREADS>;
-    t[0][4] = kb_psf_residual<13, 4, 0, false, KB_THREADS>;
-    t[0][5] = kb_psf_residual<15, 4, 0, false, KB_THREADS>;
-    t[0][6] = kb_psf_residual<17, 4, 0, false, KB_THREADS>;
-    t[0][7] = kb_psf_residual<19, 4, 0, false, KB_THREADS>;
-    t[0][8] = kb_psf_residual<21, 4, 0, false, KB_THREADS>;
-    t[0][9] = kb_psf_residual<23, 4, 0, false, KB_THREADS>;
-    t[0][10] = kb_psf_residual<25, 4, 0, false, KB_THREADS>;
-    t[0][11] = kb_psf_residual<27, 4, 0, false, KB_THREADS>;
-    t[0][12] = kb_psf_residual<29, 4, 0, false, KB_THREADS>;
-    t[0][13] = kb_psf_residual<31, 4, 0, false, KB_THREADS>;
-    t[0][14] = kb_psf_residual<33, 4, 0, false, KB_THREADS>;
-    t[1][0] = kb_psf_residual<5, 4, 1, false, KB_THREADS>;
-    t[1][1] = kb_psf_residual<7, 4, 1, false, KB_THREADS>;
-    t[1][2] = kb_psf_residual<9, 4, 1, false, KB_THREADS>;
-    t[1][3] = kb_psf_residual<11, 4, 1, false, KB_THREADS>;
-    t[1][4] = kb_psf_residual<13, 4, 1, false, KB_THREADS>;
-    t[1][5] = kb_psf_residual<15, 4, 1, false, KB_THREADS>;
-    t[1][6] = kb_psf_residual<17, 4, 1, false, KB_THREADS>;
-    t[1][7] = kb_psf_residual<19, 4, 1, false, KB_THREADS>;
-    t[1][8] = kb_psf_residual<21, 4, 1, false, KB_THREADS>;
-    t[1][9] = kb_psf_residual<23, 4, 1, false, KB_THREADS>;
-    t[1][10] = kb_psf_residual<25, 4, 1, false, KB_THREADS>;
-    t[1][11] = kb_psf_residual<27, 4, 1, false, KB_THREADS>;
-    t[1][12] = kb_psf_residual<29, 4, 1, false, KB_THREADS>;
-    t[1][13] = kb_psf_residual<31, 4, 1, false, KB_THREADS>;
-    t[1][14] = kb_psf_residual<33, 4, 1, false, KB_THREADS>;
-    t[2][0] = kb_psf_residual<5, 4, 2, false, KB_THREADS>;
-    t[2][1] = kb_psf_residual<7, 4, 2, false, KB_THREADS>;
-    t[2][2] = kb_psf_residual<9, 4, 2, false, KB_THREADS>;
-    t[2][3] = kb_psf_residual<11, 4, 2, false, KB_THREADS>;
-    t[2][4] = kb_psf_residual<13, 4, 2, false, KB_THREADS>;
-    t[2][5] = kb_psf_residual<15, 4, 2, false, KB_THREADS>;
-    t[2][6] = kb_psf_residual<17, 4, 2, false, KB_THREADS>;
-    t[2][7] = kb_psf_residual<19, 4, 2, false, KB_THREADS>;
-    t[2][8] = kb_psf_residual<21, 4, 2, false, KB_THREADS>;
-    t[2][9] = kb_psf_residual<23, 4, 2, false, KB_THREADS>;
-    t[2][10] = kb_psf_residual<25, 4, 2, false, KB_THREADS>;
-    t[2][11] = kb_psf_residual<27, 4, 2, false, KB_THREADS>;
-    t[2][12] = kb_psf_residual<29, 4, 2, false, KB_THREADS>;
-    t[2][13] = kb_psf_residual<31, 4, 2, false, KB_THREADS>;
-    t[2][14] = kb_psf_residual<33, 4, 2, false, KB_THREADS>;
+    t[(K - KB_KMIN) / 2] = kb_psf_residual<K>;
+    if constexpr (K + 2 <= KB_KMAX) fill<K + 2>(t);
 }
+
+void kb_register(KbFn* t) { fill<KB_KMIN>(t); }
 
 }  // namespace gbk

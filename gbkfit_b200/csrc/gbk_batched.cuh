@@ -27,6 +27,7 @@ struct BatchKernelArgs {
     float2* work;         // (chunk, Wz, Py, hx)
     float* model;         // optional (nsets, Nz, Ny, Nx)
     double* partials;     // (nsets, Nz, ceil(Ny / rows_k5))
+    int vec;              // Nx % 4 == 0 and obs, iw and model on 16 bytes: float4 rows
     int set0;
     // element counts of the buffers (bounds of the checked build)
     long long lim_work, lim_model, lim_part, lim_obs, lim_smem1, lim_smem5;
@@ -36,14 +37,10 @@ struct BatchKernelArgs {
     int pitch;            // row pitch of the LSF-convolved planes in HBM (floats, % 32 == 0)
     int cap;              // shared-memory floats of a PSF block (rows of one pass)
     int band, nbands;     // output rows per PSF block, bands per plane
-    int xr_slot;          // persistent PSF kernel: ints per range-entry buffer (% 4 == 0)
-    int kb_cn;            // persistent PSF kernel: sets of the launch
-    int* kb_work;         // persistent PSF kernel: item counter (zeroed before each launch)
     // FIR coefficients in the parameter block (constant bank, uniform loads)
     float vr[33];         // (K): PSF x factor, reversed, zero-padded
     float ur[33];         // (K): PSF y factor, reversed, zero-padded
     float lsfr[33];       // (Kz): LSF reversed
-    float2 ur2[33];       // (K): ur duplicated into packed pairs (FFMA2 operands)
     float* mplanes;       // (chunk, Nz, Wy, pitch): written where xr is not empty
     int nch;              // 32-column chunks per window row, ceil(Wx / 32)
     int nwfast;           // the disk's traits are exactly rpt/vpt/dpt uid 101 (smdisk_spaxel_nw)
@@ -253,21 +250,20 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf(B
 // velocities than a 32-spaxel row, so the warp's channel range (the union of
 // its lanes' output ranges) is shorter: ~1.57 instead of ~2.11 times the
 // lanes' own ranges for the 128 x 128 x 96 batch workload.  Each plane row
-// store is a 32-byte segment.  A warp's ballot of plane zo holds four rows'
-// 8-column masks; each goes into byte w of that row chunk's entry (columns
-// 8 w .. 8 w + 7) in shared memory (Nz x 4 entries, zero where no warp
-// writes), and the block stores whole entries once all four warps are done.
+// store is a 32-byte segment.  A plane's 32 lanes are four rows' 8-column
+// masks; each goes into byte w of that row chunk's entry (columns 8 w .. 8 w + 7)
+// in shared memory (Nz x 4 entries, zero where no warp writes), and the block
+// stores whole entries once all four warps are done.  The masks come after the
+// channel loop, 32 planes at once: every lane forms its output range as a
+// 32-bit row and the warp transposes the 32 rows (plane_masks32), a few
+// instructions per group instead of a ballot and its bookkeeping per plane.
 // The lines, the LSF FIR and its order of operations are those of
 // ka_lines_lsf (identical values).
-// TM (transposed masks): no ballot in the channel loop; after it, each group
-// of 32 planes gets its masks at once, every lane forming its output range
-// as a 32-bit row and the warp transposing the 32 rows (plane_masks32): the
-// same masks for a few instructions per group instead of several per plane.
 // SL (scaled line): the exponent as -t^2 with t = zf (dz s) + (z0 - v) s and
 // s = sqrt(log2(e) / (2 sigma^2)), one multiply-add and one multiply per
 // channel instead of a multiply-add, an add and two multiplies; the same line
 // up to fp32 rounding (not bit-identical to the other forms).
-template<int KZ, bool TM, bool SL = false>
+template<int KZ, bool SL>
 __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t(BatchKernelArgs P, int* status)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -311,7 +307,6 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t
     auto line = [&](int z) { return line_f(z, (float)z); };
     const bool lit = lo <= hi;
     const int olo = lit ? max(0, lo - KZ + 1) : INT_MAX, ohi = lit ? min(P.Nz - 1, hi) : -1;
-    const unsigned olen = lit ? (unsigned)(ohi - olo) : 0u;
     int zlo = olo, zhi = ohi;
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
@@ -334,8 +329,6 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t
         const long long zstride = (long long)P.Wy * P.pitch;
         float* dp = P.mplanes + ((long long)c * P.Nz * P.Wy + (row_ok ? y : 0)) * P.pitch + x +
                     zlo * zstride;
-        unsigned mm = 0u;
-        int mz = zlo, own = zlo + lane, fl = min(zlo + 31, zhi);
         float zf = (float)(zlo + KZ - 1);
         for (int zb = zlo; zb <= zhi; zb += KZ) {
 #pragma unroll
@@ -351,25 +344,12 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t
                 for (int t = 1; t < KZ; t += 2) acc1 += lz[t] * w[(k + t) % KZ];
                 if (row_ok) *dp = acc0 + acc1;      // plane zo
                 dp += zstride;
-                if constexpr (!TM) {
-                    const unsigned m = __ballot_sync(0xffffffffu,
-                                                     (unsigned)zo - (unsigned)olo <= olen);
-                    if (zo == own) mm = m;
-                    if (zo == fl) {
-                        if (own <= zo) put(own, mm);
-                        mz = zo + 1;
-                        own = mz + lane;
-                        fl = min(mz + 31, zhi);
-                    }
-                }
             }
         }
-        if constexpr (TM) {
-            // lanes without a line: olo = INT_MAX, ohi = -1 (an empty row)
-            for (int g = zlo; g <= zhi; g += 32) {
-                const unsigned m = plane_masks32(olo, ohi, g, lane);
-                if (g + lane <= zhi) put(g + lane, m);
-            }
+        // lanes without a line: olo = INT_MAX, ohi = -1 (an empty row)
+        for (int g = zlo; g <= zhi; g += 32) {
+            const unsigned m = plane_masks32(olo, ohi, g, lane);
+            if (g + lane <= zhi) put(g + lane, m);
         }
     }
     // the block's entries: every plane of its rows in the window
@@ -398,12 +378,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -414,6 +388,26 @@ __device__ __forceinline__ double sat_box(const double* T, int ld, int y0, int y
 {
     return T[(long long)y1 * ld + x1] - T[(long long)y0 * ld + x1] - T[(long long)y1 * ld + x0] +
            T[(long long)y0 * ld + x0];
+}
+
+// zeros in rows [r0, r1) of a plane outside the box of rows [y0, y1) and columns
+// [x0, x1) (x0 a multiple of 8, x1 a multiple of 8 or nx); a warp per row
+__device__ __forceinline__ void kb_zero_rows(float* m, int nx, bool vec, int r0, int r1, int y0, int y1,
+                                             int x0, int x1, int warp, int lane, int nwarps)
+{
+    for (int y = r0 + warp; y < r1; y += nwarps) {
+        float* row = m + (long long)y * nx;
+        const bool in = y >= y0 && y < y1;
+        const int a = in ? x0 : nx, e = in ? x1 : nx;      // zero [0, a) and [e, nx)
+        if (vec) {
+            for (int x = 4 * lane; x < nx; x += 128)
+                if (x < a || x >= e)
+                    *reinterpret_cast<float4*>(row + x) = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            for (int x = lane; x < nx; x += 32)
+                if (x < a || x >= e) row[x] = 0.f;
+        }
+    }
 }
 
 // KB: one block per (set, output plane zo, band of output rows), sets fastest.  The block
@@ -431,84 +425,35 @@ __device__ __forceinline__ double sat_box(const double* T, int ld, int y0, int y
 constexpr int KB_THREADS = 128;
 constexpr int KB_NX_MAX = 512;  // widest data cube of the direct mode
 
-// MINB: resident blocks per SM the registers are sized for (4: up to 128
-// registers a thread; 5: up to 102, with the shared memory per block sized to
-// match, see setup_direct)
-// EPI: how the y FIR meets the residual.  0: y FIR in place in rounds of
-// items with a barrier between loads and stores, then a residual pass over the
-// pass's rows reading shared memory; 1: the residual in each y-FIR item's
-// epilogue (no write-back, no barriers between items), its data loaded after
-// the item's FIR; 2: as 1, with the item's data requested before its FIR.
-template<int K, int MINB, int EPI, bool PF, int NT>
-__global__ void __launch_bounds__(NT, MINB) kb_psf_residual(BatchKernelArgs P)
+template<int K>
+__global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs P)
 {
     constexpr int NW = (K + 7 + 3) / 4;     // float4 slots of one 8-output x window
-    constexpr int NWARPS = NT / 32;
+    constexpr int NT = KB_THREADS, NWARPS = NT / 32;
     extern __shared__ float4 sm4[];
     float* S = reinterpret_cast<float*>(sm4);                   // (rows of a pass, bp)
-    // (in1 - ob0, nch) range entries of an item; PF: two buffers of xr_slot ints
-    int* const s_xr0 = reinterpret_cast<int*>(S + P.cap);
+    int* const s_xr = reinterpret_cast<int*>(S + P.cap);        // (in1 - ob0, nch) range entries
     __shared__ float warp_part[NWARPS];
     __shared__ int s_box[4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ld = P.Nx + 1;
-    // PF (persistent): the blocks take items of cn x Nz x nbands (sets fastest)
-    // from a work counter, one ahead: the next item's range entries are copied
-    // into the other buffer (cp.async) while this item runs.  Otherwise one
-    // item per block:
-    // blockIdx.x the set, blockIdx.y the (plane, band) - sets vary fastest, so
-    // the blocks in flight share a few planes of the data.
-    const int nit = PF ? P.kb_cn * P.Nz * P.nbands : 1;
-    auto entries = [&](int it, const int*& src, int& n, int& ob0_) {
-        const int c_ = PF ? it % P.kb_cn : blockIdx.x;
-        const int yi = PF ? it / P.kb_cn : blockIdx.y;
-        const int zo_ = yi / P.nbands, band_ = yi % P.nbands;
-        ob0_ = band_ * P.band;
-        const int ob1_ = min(P.Ny, ob0_ + P.band), in1_ = min(P.Wy, ob1_ + K - 1);
-        src = P.xrt + (((long long)c_ * P.Nz + zo_) * P.Wy + ob0_) * P.nch;
-        n = (in1_ - ob0_) * P.nch;
-    };
-    auto prefetch = [&](int it, int* dst) {
-        const int* src;
-        int n, o;
-        entries(it, src, n, o);
-        for (int i = threadIdx.x; i < n; i += NT) cp_async4(dst + i, src + i);
-    };
-    __shared__ int s_next;
-    int buf = 0, it = 0;
-    if (PF) {
-        if (threadIdx.x == 0) s_next = atomicAdd(P.kb_work, 1);
-        __syncthreads();
-        it = s_next;
-        __syncthreads();      // every thread has read s_next before it is rewritten
-        if (it < nit) prefetch(it, s_xr0);
-    }
-    while (it < nit) {
-    int* const s_xr = s_xr0 + buf * P.xr_slot;
-    const int c = PF ? it % P.kb_cn : (int)blockIdx.x, b = P.set0 + c;
-    const int yi = PF ? it / P.kb_cn : (int)blockIdx.y;
-    const int zo = yi / P.nbands, band = yi % P.nbands;
+    // blockIdx.x the set, blockIdx.y the (plane, band): sets vary fastest, so
+    // the blocks in flight share a few planes of the data
+    const int c = blockIdx.x, b = P.set0 + c;
+    const int zo = blockIdx.y / P.nbands, band = blockIdx.y % P.nbands;
     const int ob0 = band * P.band, ob1 = min(P.Ny, ob0 + P.band);  // output rows [ob0, ob1)
     const int in1 = min(P.Wy, ob1 + K - 1);                        // input rows [ob0, in1)
     const long long prow = ((long long)c * P.Nz + zo) * P.Wy;
     const int* xr = P.xrt + prow * P.nch;                          // (y, chunk) at [y nch + chunk]
     const double* T = P.sat + (long long)zo * (P.Ny + 1) * ld;
-    if (PF) cp_async_wait_all();          // this item's entries (this thread's copies)
     if (threadIdx.x == 0) {
         s_box[0] = INT_MAX; s_box[1] = -1; s_box[2] = INT_MAX; s_box[3] = -1;
-        if (PF) s_next = atomicAdd(P.kb_work, 1);
     }
     __syncthreads();
-    // the next item's entries, into the other buffer (its last reader, the
-    // item before this one, has finished)
-    const int next = PF ? s_next : nit;
-    if (PF && next < nit) prefetch(next, s_xr0 + (buf ^ 1) * P.xr_slot);
-    do {
     // bounding box of the nonzero input row chunks
     {
         int y0 = INT_MAX, y1 = -1, x0 = INT_MAX, x1 = -1;
         // the entries of rows [ob0, in1), eight loads in flight per thread
-        // (PF: already in s_xr)
         const int* src = xr + ob0 * P.nch;
         const int n = (in1 - ob0) * P.nch;
         for (int i0 = 0; i0 < n; i0 += 8 * NT) {
@@ -516,12 +461,8 @@ __global__ void __launch_bounds__(NT, MINB) kb_psf_residual(BatchKernelArgs P)
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int i = i0 + u * NT + threadIdx.x;
-                if (PF) {
-                    v[u] = i < n ? s_xr[i] : 0;
-                } else {
-                    v[u] = i < n ? src[i] : 0;
-                    if (i < n) s_xr[i] = v[u];
-                }
+                v[u] = i < n ? src[i] : 0;
+                if (i < n) s_xr[i] = v[u];
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -556,11 +497,9 @@ __global__ void __launch_bounds__(NT, MINB) kb_psf_residual(BatchKernelArgs P)
     const long long part = ((long long)b * P.Nz + zo) * P.nbands + band;
     if (y1 < 0) {   // nothing reaches this band: the model is 0 on it
         if (model)
-            for (long long i = (long long)ob0 * P.Nx + threadIdx.x; i < (long long)ob1 * P.Nx;
-                 i += NT)
-                model[i] = 0.f;
+            kb_zero_rows(model, P.Nx, P.vec, ob0, ob1, ob0, ob0, 0, 0, warp, lane, NWARPS);
         if (threadIdx.x == 0) P.partials[part] = sat_box(T, ld, ob0, ob1, 0, P.Nx);
-        break;
+        return;
     }
     // output box: x in 8-column strips [g_lo, g_hi], rows [yo_lo, yb_end) in 8-row groups
     const int g_lo = max(0, x0 - K + 1) >> 3, g_hi = min(P.Nx - 1, x1) >> 3;
@@ -677,221 +616,110 @@ __global__ void __launch_bounds__(NT, MINB) kb_psf_residual(BatchKernelArgs P)
             }
         }
         __syncthreads();
-        if constexpr (EPI == 0) {
-            constexpr int kIt = 1;     // y items per thread and round
-            // y FIR in place: model(yo, xo) = sum_t ur[t] S[yo + t][xo], written to S row yo.
-            // Packed FP32 pairs (FFMA2: two lanes of fma, each rounded as fmaf),
-            // columns (x, x+1) and (x+2, x+3) of a float4 per instruction.  Items
-            // (8-row group, float4 column) in ascending order, NT x kIt
-            // per round, loads before the round's barrier and stores after it: a
-            // column's group is written only after every lower group of that
-            // column, the only readers of its rows, has loaded them.
-            {
-                float2 u2[K];
-    #pragma unroll
-                for (int t = 0; t < K; ++t) u2[t] = make_float2(P.ur[t], P.ur[t]);
-                const int nitems = ng * ns4;
-                for (int gr0 = 0; gr0 < nitems; gr0 += NT * kIt) {
-                    float2 acc[kIt][8][2];
-    #pragma unroll
-                    for (int it = 0; it < kIt; ++it) {
-                        const int item = gr0 + threadIdx.x + it * NT;
-    #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            acc[it][q][0] = make_float2(0.f, 0.f);
-                            acc[it][q][1] = make_float2(0.f, 0.f);
-                        }
-                        if (item < nitems) {
-                            const int rb = 8 * (item / ns4), s4 = item % ns4;
-                            const float4* colp = reinterpret_cast<const float4*>(S) + rb * bp4 + s4;
-    #pragma unroll
-                            for (int m = 0; m < K + 7; ++m) {
-                                const float4 p = colp[m * bp4];
-                                const float2 pxy = make_float2(p.x, p.y), pzw = make_float2(p.z, p.w);
-    #pragma unroll
-                                for (int q = 0; q < 8; ++q) {
-                                    const int t = m - q;
-                                    if (t >= 0 && t < K) {
-                                        acc[it][q][0] = __ffma2_rn(u2[t], pxy, acc[it][q][0]);
-                                        acc[it][q][1] = __ffma2_rn(u2[t], pzw, acc[it][q][1]);
-                                    }
-                                }
-                            }
-                        }
-                    }
-                    __syncthreads();
-    #pragma unroll
-                    for (int it = 0; it < kIt; ++it) {
-                        const int item = gr0 + threadIdx.x + it * NT;
-                        if (item < nitems) {
-                            const int rb = 8 * (item / ns4), s4 = item % ns4;
-    #pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                if (ys + rb + q < ye)
-                                    reinterpret_cast<float4*>(S)[(rb + q) * bp4 + s4] =
-                                        make_float4(acc[it][q][0].x, acc[it][q][0].y,
-                                                    acc[it][q][1].x, acc[it][q][1].y);
-                        }
-                    }
-                    __syncthreads();
+        // y FIR in place: model(yo, xo) = sum_t ur[t] S[yo + t][xo], written to S row yo.
+        // Packed FP32 pairs (FFMA2: two lanes of fma, each rounded as fmaf),
+        // columns (x, x+1) and (x+2, x+3) of a float4 per instruction.  Items
+        // (8-row group, float4 column) in ascending order, NT per round, loads
+        // before the round's barrier and stores after it: a column's group is
+        // written only after every lower group of that column, the only
+        // readers of its rows, has loaded them.
+        {
+            float2 u2[K];
+#pragma unroll
+            for (int t = 0; t < K; ++t) u2[t] = make_float2(P.ur[t], P.ur[t]);
+            const int nitems = ng * ns4;
+            for (int gr0 = 0; gr0 < nitems; gr0 += NT) {
+                float2 acc[8][2];
+                const int item = gr0 + threadIdx.x;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    acc[q][0] = make_float2(0.f, 0.f);
+                    acc[q][1] = make_float2(0.f, 0.f);
                 }
-            }
-            // crop + residual over rows [ys, ye), columns [xb0, xb_end)
-            if ((P.Nx & 3) == 0) {
-                // flat float4 index over the pass, stepped without divisions
-                const int nv = (xb_end - xb0) >> 2;        // xb0 and xb_end are multiples of 4
-                const int n = (ye - ys) * nv;
-                const int dq = NT / nv, dr = NT % nv;
-                int row = threadIdx.x / nv, col = threadIdx.x % nv;
-                // running offsets: si in S (float4), vi in the data plane (float)
-                int si = row * bp4 + col, vi = pbase + (ys + row) * P.Nx + xb0 + 4 * col;
-                const int dsi = dq * bp4 + dr, dvi = dq * P.Nx + 4 * dr;
-                float2 s2 = make_float2(0.f, 0.f);
-    #pragma unroll 4
-                for (int i = threadIdx.x; i < n; i += NT) {
-                    const float4 m = reinterpret_cast<const float4*>(S)[si];
-                    const float4 o = *reinterpret_cast<const float4*>(P.obs + vi);
-                    const float4 w = *reinterpret_cast<const float4*>(P.iw + vi);
-                    // packed pairs: r = (m - o) w, s2 += r^2
-                    const float2 r01 = __fmul2_rn(__fadd2_rn(make_float2(m.x, m.y),
-                                                             make_float2(-o.x, -o.y)),
-                                                  make_float2(w.x, w.y));
-                    const float2 r23 = __fmul2_rn(__fadd2_rn(make_float2(m.z, m.w),
-                                                             make_float2(-o.z, -o.w)),
-                                                  make_float2(w.z, w.w));
-                    s2 = __ffma2_rn(r01, r01, s2);
-                    s2 = __ffma2_rn(r23, r23, s2);
-                    if (model) *reinterpret_cast<float4*>(model + (vi - pbase)) = m;
-                    col += dr;
-                    si += dsi;
-                    vi += dvi;
-                    if (col >= nv) {
-                        col -= nv;
-                        si += bp4 - nv;
-                        vi += P.Nx - 4 * nv;
-                    }
-                }
-                sum += s2.x + s2.y;
-            } else {
-                const int nw = xb_end - xb0, n = (ye - ys) * nw;
-                for (int i = threadIdx.x; i < n; i += NT) {
-                    const int row = i / nw, col = i % nw;
-                    const int yo = ys + row, xo = xb0 + col;
-                    const float m = S[row * bp + col];
-                    const int vi = pbase + yo * P.Nx + xo;
-                    const float r0 = (m - P.obs[vi]) * P.iw[vi];
-                    sum += r0 * r0;
-                    if (model) model[yo * P.Nx + xo] = m;
-                }
-            }
-        } else {
-            // y FIR with the residual in its epilogue: item (8-row group rb, float4
-            // column s4) computes model(ys + rb + q, xb0 + 4 s4 + j) = sum_t ur[t]
-            // S[rb + q + t][4 s4 + j] for q < 8, j < 4 in registers, on packed FP32
-            // pairs (FFMA2: two lanes of fma, each rounded as fmaf), then compares
-            // them with the data (crop + residual, objective.hpp:7-31) and adds
-            // r^2.  S is only read here, so items need no barriers between them.
-            {
-                const int nitems = ng * ns4;
-                const bool vec = (P.Nx & 3) == 0;
-                float2 s2 = make_float2(0.f, 0.f);
-                for (int item = threadIdx.x; item < nitems; item += NT) {
-                    const int rb = 8 * (item / ns4), s4 = item % ns4;
-                    float2 acc[8][2];
-    #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        acc[q][0] = make_float2(0.f, 0.f);
-                        acc[q][1] = make_float2(0.f, 0.f);
-                    }
-                    const int xo = xb0 + 4 * s4;
-                    const bool inside = xo < xb_end;
-                    // the item's data and weights, requested before its FIR so that
-                    // their loads are in flight while the multiply-adds run
-                    // (Nx % 4 == 0: a float4 column lies wholly inside or outside the crop)
-                    float4 ov[8], wv[8];
-                    if (EPI == 2 && vec) {
-    #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int yo = ys + rb + q;
-                            if (inside && yo < ye) {
-                                const int vi = pbase + yo * P.Nx + xo;
-                                ov[q] = __ldg(reinterpret_cast<const float4*>(P.obs + vi));
-                                wv[q] = __ldg(reinterpret_cast<const float4*>(P.iw + vi));
-                            } else {
-                                ov[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                wv[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            }
-                        }
-                    }
+                const int rb = 8 * (item / ns4), s4 = item % ns4;
+                if (item < nitems) {
                     const float4* colp = reinterpret_cast<const float4*>(S) + rb * bp4 + s4;
-    #pragma unroll
+#pragma unroll
                     for (int m = 0; m < K + 7; ++m) {
                         const float4 p = colp[m * bp4];
                         const float2 pxy = make_float2(p.x, p.y), pzw = make_float2(p.z, p.w);
-    #pragma unroll
+#pragma unroll
                         for (int q = 0; q < 8; ++q) {
                             const int t = m - q;
                             if (t >= 0 && t < K) {
-                                acc[q][0] = __ffma2_rn(P.ur2[t], pxy, acc[q][0]);
-                                acc[q][1] = __ffma2_rn(P.ur2[t], pzw, acc[q][1]);
-                            }
-                        }
-                    }
-                    if (!inside) continue;
-                    if (vec) {
-    #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int yo = ys + rb + q;
-                            if (yo >= ye) break;
-                            const int vi = pbase + yo * P.Nx + xo;
-                            float4 o, w;
-                            if constexpr (EPI == 2) {
-                                o = ov[q];
-                                w = wv[q];
-                            } else {
-                                o = __ldg(reinterpret_cast<const float4*>(P.obs + vi));
-                                w = __ldg(reinterpret_cast<const float4*>(P.iw + vi));
-                            }
-                            const float2 r01 = __fmul2_rn(__fadd2_rn(acc[q][0], make_float2(-o.x, -o.y)),
-                                                          make_float2(w.x, w.y));
-                            const float2 r23 = __fmul2_rn(__fadd2_rn(acc[q][1], make_float2(-o.z, -o.w)),
-                                                          make_float2(w.z, w.w));
-                            s2 = __ffma2_rn(r01, r01, s2);
-                            s2 = __ffma2_rn(r23, r23, s2);
-                            if (model)
-                                *reinterpret_cast<float4*>(model + (vi - pbase)) =
-                                    make_float4(acc[q][0].x, acc[q][0].y, acc[q][1].x, acc[q][1].y);
-                        }
-                    } else {
-    #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            const int yo = ys + rb + q;
-                            if (yo >= ye) break;
-                            const float mv[4] = {acc[q][0].x, acc[q][0].y, acc[q][1].x, acc[q][1].y};
-    #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                if (xo + j >= xb_end) break;
-                                const int vi = pbase + yo * P.Nx + xo + j;
-                                const float r0 = (mv[j] - P.obs[vi]) * P.iw[vi];
-                                s2.x = fmaf(r0, r0, s2.x);
-                                if (model) model[yo * P.Nx + xo + j] = mv[j];
+                                acc[q][0] = __ffma2_rn(u2[t], pxy, acc[q][0]);
+                                acc[q][1] = __ffma2_rn(u2[t], pzw, acc[q][1]);
                             }
                         }
                     }
                 }
-                sum += s2.x + s2.y;
+                __syncthreads();
+                if (item < nitems) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (ys + rb + q < ye)
+                            reinterpret_cast<float4*>(S)[(rb + q) * bp4 + s4] =
+                                make_float4(acc[q][0].x, acc[q][0].y, acc[q][1].x, acc[q][1].y);
+                }
+                __syncthreads();
+            }
+        }
+        // crop + residual over rows [ys, ye), columns [xb0, xb_end)
+        if (P.vec) {
+            // flat float4 index over the pass, stepped without divisions
+            const int nv = (xb_end - xb0) >> 2;        // xb0 and xb_end are multiples of 4
+            const int n = (ye - ys) * nv;
+            const int dq = NT / nv, dr = NT % nv;
+            int row = threadIdx.x / nv, col = threadIdx.x % nv;
+            // running offsets: si in S (float4), vi in the data plane (float)
+            int si = row * bp4 + col, vi = pbase + (ys + row) * P.Nx + xb0 + 4 * col;
+            const int dsi = dq * bp4 + dr, dvi = dq * P.Nx + 4 * dr;
+            float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n; i += NT) {
+                const float4 m = reinterpret_cast<const float4*>(S)[si];
+                const float4 o = *reinterpret_cast<const float4*>(P.obs + vi);
+                const float4 w = *reinterpret_cast<const float4*>(P.iw + vi);
+                // packed pairs: r = (m - o) w, s2 += r^2
+                const float2 r01 = __fmul2_rn(__fadd2_rn(make_float2(m.x, m.y),
+                                                         make_float2(-o.x, -o.y)),
+                                              make_float2(w.x, w.y));
+                const float2 r23 = __fmul2_rn(__fadd2_rn(make_float2(m.z, m.w),
+                                                         make_float2(-o.z, -o.w)),
+                                              make_float2(w.z, w.w));
+                s2 = __ffma2_rn(r01, r01, s2);
+                s2 = __ffma2_rn(r23, r23, s2);
+                if (model) *reinterpret_cast<float4*>(model + (vi - pbase)) = m;
+                col += dr;
+                si += dsi;
+                vi += dvi;
+                if (col >= nv) {
+                    col -= nv;
+                    si += bp4 - nv;
+                    vi += P.Nx - 4 * nv;
+                }
+            }
+            sum += s2.x + s2.y;
+        } else {
+            // rows of any alignment: a warp per row, lanes along it
+            const int nw = xb_end - xb0;
+            for (int row = warp; row < ye - ys; row += NWARPS) {
+                const float* m = S + row * bp;
+                const int v0 = pbase + (ys + row) * P.Nx + xb0;
+                const float *od = P.obs + v0, *iw = P.iw + v0;
+                float* md = model ? model + (v0 - pbase) : nullptr;
+#pragma unroll 4
+                for (int x = lane; x < nw; x += 32) {
+                    const float r0 = (m[x] - od[x]) * iw[x];
+                    sum += r0 * r0;
+                    if (md) md[x] = m[x];
+                }
             }
         }
         __syncthreads();    // S is reloaded by the next pass
     }
-    if (model) {
-        const int bw = P.Nx;
-        for (long long i = (long long)ob0 * bw + threadIdx.x; i < (long long)ob1 * bw;
-             i += NT) {
-            const int yo = (int)(i / bw), xo = (int)(i % bw);
-            if (yo < yo_lo || yo >= yb_end || xo < xb0 || xo >= xb_end) model[i] = 0.f;
-        }
-    }
+    if (model)
+        kb_zero_rows(model, P.Nx, P.vec, ob0, ob1, yo_lo, yb_end, xb0, xb_end, warp, lane, NWARPS);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0) warp_part[warp] = sum;
@@ -906,148 +734,6 @@ __global__ void __launch_bounds__(NT, MINB) kb_psf_residual(BatchKernelArgs P)
             atomicAdd(&P.counters[GBK_CTR_KB_VOX], c_v);
         }
     }
-    } while (0);
-    if (PF) __syncthreads();   // before the next item reuses the shared memory
-    buf ^= 1;
-    it = next;
-    }
-}
-
-// ka_lines_lsf on two 32-column chunks per warp: lane l evaluates columns
-// 64 q + l and 64 q + 32 + l (chunks 2 q and 2 q + 1) and runs both LSF FIRs
-// as packed FP32 pairs (FFMA2: two lanes of fma, each rounded as fmaf, so
-// every value is the one ka_lines_lsf computes); each chunk keeps its own
-// range-table entries.  Half the multiply-add instructions per spaxel.
-template<int KZ>
-__global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 5 : 4)) ka_lines_lsf2(BatchKernelArgs P, int* status)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int npair = (P.nch + 1) >> 1;
-    const int item = blockIdx.x * (KA_THREADS / 32) + warp;
-    if (item >= P.Wy * npair) return;                    // whole warp
-    const int y = item / npair, c0 = 2 * (item % npair), c1 = c0 + 1;
-    const bool has1 = c1 < P.nch;                        // warp-uniform
-    const int c = blockIdx.y, b = P.set0 + c;
-    const DiskArgs a = set_disk(P, b);
-    const DiskConst kc = disk_const(a);
-    int bad = 0;
-    float amp[2], rinv[2], vv[2];
-    int lo[2], hi[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int x = (c0 + h) * 32 + lane;
-        SpaxelOut o{};
-        lo[h] = INT_MAX;
-        hi[h] = -1;
-        amp[h] = 0.f;
-        rinv[h] = 0.f;
-        const bool on = x < P.Wx && (P.nwfast ? smdisk_spaxel_nw(a, kc, x, y, o)
-                                               : smdisk_spaxel(a, kc, x, y, 0, o, bad));
-        if (on && line_window(o.vv, o.dv, P.Wz, a.spec_step, a.spec_zero, lo[h], hi[h])) {
-            amp[h] = o.orv * (1 / (o.dv * sqrtf(2 * GBK_PI)));
-            rinv[h] = 1.4426950408889634f / (2 * o.dv * o.dv);
-        } else {
-            lo[h] = INT_MAX;
-            hi[h] = -1;
-        }
-        vv[h] = o.vv;
-    }
-    const float z0 = a.spec_zero, dz = a.spec_step;
-    const unsigned wlen0 = (unsigned)hi[0] - (unsigned)lo[0];
-    const unsigned wlen1 = (unsigned)hi[1] - (unsigned)lo[1];
-    // the lines of both columns at window channel z (as line_f of ka_lines_lsf)
-    auto line2 = [&](int z, float zf) {
-        const float zv = z0 + zf * dz;
-        const float d0 = zv - vv[0], d1 = zv - vv[1];
-        float e0, e1;
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(-(d0 * d0) * rinv[0]));
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(-(d1 * d1) * rinv[1]));
-        return make_float2((unsigned)z - (unsigned)lo[0] <= wlen0 ? amp[0] * e0 : 0.f,
-                           (unsigned)z - (unsigned)lo[1] <= wlen1 ? amp[1] * e1 : 0.f);
-    };
-    int olo[2], ohi[2];
-    unsigned olen[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const bool lit = lo[h] <= hi[h];
-        olo[h] = lit ? max(0, lo[h] - KZ + 1) : INT_MAX;
-        ohi[h] = lit ? min(P.Nz - 1, hi[h]) : -1;
-        olen[h] = lit ? (unsigned)(ohi[h] - olo[h]) : 0u;
-    }
-    int zlo = min(olo[0], olo[1]), zhi = max(ohi[0], ohi[1]);
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        zlo = min(zlo, __shfl_xor_sync(0xffffffffu, zlo, s));
-        zhi = max(zhi, __shfl_xor_sync(0xffffffffu, zhi, s));
-    }
-    // the range table, plane-major: the chunks' entries of plane z at [z * xs]
-    const long long xs = (long long)P.Wy * P.nch;
-    int* xr0 = P.xrt + ((long long)c * P.Nz * P.Wy + y) * P.nch + c0;
-    int* xr1 = xr0 + 1;                                   // chunk c1 (used when has1)
-    for (int zo = lane; zo < P.Nz; zo += 32)
-        if (zo < zlo || zo > zhi) {
-            xr0[zo * xs] = 0;
-            if (has1) xr1[zo * xs] = 0;
-        }
-    if (zlo <= zhi) {
-        float2 lz[KZ];
-#pragma unroll
-        for (int t = 0; t < KZ; ++t) lz[t] = make_float2(P.lsfr[t], P.lsfr[t]);
-        float2 w[KZ];
-#pragma unroll
-        for (int t = 0; t < KZ - 1; ++t) w[t] = line2(zlo + t, (float)(zlo + t));
-        const long long zstride = (long long)P.Wy * P.pitch;
-        float* dp = P.mplanes + ((long long)c * P.Nz * P.Wy + y) * P.pitch + c0 * 32 + lane +
-                    zlo * zstride;
-        unsigned mm0 = 0u, mm1 = 0u;
-        int mz = zlo, own = zlo + lane, fl = min(zlo + 31, zhi);
-        float zf = (float)(zlo + KZ - 1);
-        for (int zb = zlo; zb <= zhi; zb += KZ) {
-#pragma unroll
-            for (int k = 0; k < KZ; ++k) {
-                const int zo = zb + k;
-                if (zo > zhi) break;
-                w[(k + KZ - 1) % KZ] = line2(zo + KZ - 1, zf);
-                zf += 1.f;
-                float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int t = 0; t < KZ; t += 2) acc0 = __ffma2_rn(lz[t], w[(k + t) % KZ], acc0);
-#pragma unroll
-                for (int t = 1; t < KZ; t += 2) acc1 = __ffma2_rn(lz[t], w[(k + t) % KZ], acc1);
-                const float2 r = __fadd2_rn(acc0, acc1);
-                dp[0] = r.x;
-                if (has1) dp[32] = r.y;
-                dp += zstride;
-                const unsigned m0 = __ballot_sync(0xffffffffu,
-                                                  (unsigned)zo - (unsigned)olo[0] <= olen[0]);
-                const unsigned m1 = __ballot_sync(0xffffffffu,
-                                                  (unsigned)zo - (unsigned)olo[1] <= olen[1]);
-                if (zo == own) {
-                    mm0 = m0;
-                    mm1 = m1;
-                }
-                if (zo == fl) {
-                    if (own <= zo) {
-                        xr0[own * xs] = (int)mm0;
-                        if (has1) xr1[own * xs] = (int)mm1;
-                    }
-                    mz = zo + 1;
-                    own = mz + lane;
-                    fl = min(mz + 31, zhi);
-                }
-            }
-        }
-    }
-    if (P.counters && lane == 0) {
-        const unsigned long long nc = has1 ? 2 : 1;
-        atomicAdd(&P.counters[GBK_CTR_KA_SPAXEL], 32ull * nc);
-        if (zlo <= zhi) {
-            const unsigned long long n = (unsigned long long)(zhi - zlo + 1) * 32 * nc;
-            atomicAdd(&P.counters[GBK_CTR_KA_FMA], n * KZ);
-            atomicAdd(&P.counters[GBK_CTR_KA_LINE], n + (KZ - 1) * 32ull * nc);
-        }
-    }
-    if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
 }
 
 // The LSF FIR of given model cubes (any gmodel's output on the evaluation
@@ -1120,20 +806,12 @@ static_assert(KA_KMAX <= 33 && KB_KMAX <= 33, "coefficient arrays of BatchKernel
 // fill t[Kz / 2] (model kernel) and t[(K - KB_KMIN) / 2] (PSF kernel)
 void ka_register_short(KaFn* t);
 void ka_register_long(KaFn* t);
-// t[Kz / 2]: the two-chunk model kernel (ka_lines_lsf2)
-void ka2_register(KaFn* t);
 // t[Kz / 2]: the model kernel on 4 x 8 spaxel tiles (ka_lines_lsf_t)
-void ka_t_register(KaFn* t, bool tm, bool sl);
+void ka_t_register(KaFn* t, bool sl);
 // t[Kz / 2]: the LSF FIR of given model cubes
 typedef void (*KcFn)(BatchKernelArgs, const float*);
 void kc_register(KcFn* t);
-// t[v][(K - KB_KMIN) / 2] for the PSF kernel variant v = 3 * (MINB == 5) + EPI
-// (v = 6: MINB 4, EPI 0, persistent with prefetched range entries; v = 7:
-// 256-thread blocks, MINB 2, EPI 0)
-constexpr int KB_VARIANTS = 8;
-void kb_register4(KbFn (*t)[(KB_KMAX - KB_KMIN) / 2 + 1]);   // MINB 4, EPI 0-2
-void kb_register5(KbFn (*t)[(KB_KMAX - KB_KMIN) / 2 + 1]);   // MINB 5, EPI 0-2
-void kb_register_pf(KbFn (*t)[(KB_KMAX - KB_KMIN) / 2 + 1]); // MINB 4, EPI 0, persistent
-void kb_register_wide(KbFn (*t)[(KB_KMAX - KB_KMIN) / 2 + 1]); // 256 threads, MINB 2, EPI 0
+// t[(K - KB_KMIN) / 2]: the PSF kernel
+void kb_register(KbFn* t);
 
 }  // namespace gbk

@@ -31,6 +31,7 @@ constexpr int KP_MAX_W = 384;         // longest window: 24 row groups, 12 chunk
 
 struct PlaneArgs {
     int Nx, Ny, Nz, Wx, Wy, nch, pitch;    // pitch: of the planes (floats)
+    int vec;                               // as BatchKernelArgs::vec
     int hxp, ngw, set0;                    // padded spectrum columns; window row groups
     const float* mplanes;                  // (sets, Nz, Wy, pitch)
     const int* xrt;                        // (sets, Nz, Wy, nch)
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(KP_P * (N1 > 16 ? N1 : 16)) kp_resid(PlaneArgs
         const float* od = P.obs + v0 + (long long)lr * P.Nx;
         const float* iw = P.iw + v0 + (long long)lr * P.Nx;
         float* md = model ? model + (long long)lr * P.Nx : nullptr;
-        if ((P.Nx & 3) == 0) {
+        if (P.vec) {
             // the rows start on 16 bytes
             for (int x = 4 * c; x < P.Nx; x += 4 * KP_L) {
                 const float4 o = __ldg(reinterpret_cast<const float4*>(od + x));
