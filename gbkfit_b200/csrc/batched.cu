@@ -531,7 +531,7 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     if (P.K > KB_KMAX || P.Kz > KA_KMAX || P.Nx > KB_NX_MAX || P.Wx > 1024 ||
         (long long)P.Nx * P.Ny * P.Nz >= (1LL << 31))
         return GBKB200_ERR_UNSUPPORTED;
-    const int NW = (P.K + 7 + 3) / 4;
+    const int NW = (P.K + KB_XS - 1 + 3) / 4;
     P.pitch = (P.Wx + 31) / 32 * 32;
     P.nch = (P.Wx + 31) / 32;
     P.nwfast = nodewise(d) ? 1 : 0;
@@ -541,7 +541,7 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     // shared memory of a PSF block: rows of one pass at the widest box pitch;
     // at least K + 15 rows (8 output rows a pass), at most the whole band,
     // otherwise 54 KB (four blocks per SM)
-    int bpmax = 4 * (2 * ((P.Nx + 7) / 8 - 1) + NW);
+    int bpmax = 4 * (KB_XS / 4 * (((P.Nx + 3) / 4 + KB_XS / 4 - 1) / (KB_XS / 4) - 1) + NW);
     bpmax += ((4 - bpmax % 32) + 32) % 32;
     // range entries of the band's input rows
     const long long xr_bytes = (long long)(P.band + P.K - 1) * P.nch * sizeof(int);

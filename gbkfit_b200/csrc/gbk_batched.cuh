@@ -372,10 +372,13 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t
     if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
+// 16-byte copy to shared memory, or 16 zero bytes (gmem is not read then)
+__device__ __forceinline__ void cp_async16_or_zero(void* smem, const void* gmem, bool on)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
+                 "r"(on ? 16 : 0)
+                 : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all()
@@ -391,7 +394,7 @@ __device__ __forceinline__ double sat_box(const double* T, int ld, int y0, int y
 }
 
 // zeros in rows [r0, r1) of a plane outside the box of rows [y0, y1) and columns
-// [x0, x1) (x0 a multiple of 8, x1 a multiple of 8 or nx); a warp per row
+// [x0, x1) (multiples of 4, x1 possibly nx); a warp per row
 __device__ __forceinline__ void kb_zero_rows(float* m, int nx, bool vec, int r0, int r1, int y0, int y1,
                                              int x0, int x1, int warp, int lane, int nwarps)
 {
@@ -417,18 +420,19 @@ __device__ __forceinline__ void kb_zero_rows(float* m, int nx, bool vec, int r0,
 //   - the rows' nonzero 4-column groups are loaded from HBM (cp.async), the rest of
 //     the rows that the y FIR reads is zeroed;
 //   - x FIR in place, a warp per row, its lanes on consecutive (row, strip)
-//     pairs of its rows, 8 outputs per lane window;
+//     pairs of its rows, 12 outputs per lane window;
 //   - y FIR, 8 x 4 outputs per (8-row group, column) item in registers, and
 //     in the same item the crop, residual (objective.hpp:7-31) and r^2
 //     against the data.
 // The zero-model residual outside the box comes from the summed-area table.
 constexpr int KB_THREADS = 128;
+constexpr int KB_XS = 12;       // output columns of an x FIR strip
 constexpr int KB_NX_MAX = 512;  // widest data cube of the direct mode
 
 template<int K>
 __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs P)
 {
-    constexpr int NW = (K + 7 + 3) / 4;     // float4 slots of one 8-output x window
+    constexpr int NW = (K + KB_XS - 1 + 3) / 4;     // float4 slots of one x window
     constexpr int NT = KB_THREADS, NWARPS = NT / 32;
     extern __shared__ float4 sm4[];
     float* S = reinterpret_cast<float*>(sm4);                   // (rows of a pass, bp)
@@ -450,39 +454,33 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         s_box[0] = INT_MAX; s_box[1] = -1; s_box[2] = INT_MAX; s_box[3] = -1;
     }
     __syncthreads();
-    // bounding box of the nonzero input row chunks
+    // bounding box of the nonzero input row chunks: a thread per row
     {
         int y0 = INT_MAX, y1 = -1, x0 = INT_MAX, x1 = -1;
-        // the entries of rows [ob0, in1), eight loads in flight per thread
-        const int* src = xr + ob0 * P.nch;
-        const int n = (in1 - ob0) * P.nch;
-        for (int i0 = 0; i0 < n; i0 += 8 * NT) {
-            int v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = i0 + u * NT + threadIdx.x;
-                v[u] = i < n ? src[i] : 0;
-                if (i < n) s_xr[i] = v[u];
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (v[u] != 0) {
-                    const int i = i0 + u * NT + (int)threadIdx.x;
-                    const int r = i / P.nch, ch = i - r * P.nch;
-                    y0 = min(y0, ob0 + r);
-                    y1 = max(y1, ob0 + r);
-                    x0 = min(x0, ch * 32 + __ffs(v[u]) - 1);
-                    x1 = max(x1, ch * 32 + 31 - __clz(v[u]));
+        for (int r = threadIdx.x; r < in1 - ob0; r += NT) {
+            const int* src = xr + (ob0 + r) * P.nch;
+            int* dst = s_xr + r * P.nch;
+            int first = INT_MAX, last = -1;
+#pragma unroll 4
+            for (int ch = 0; ch < P.nch; ++ch) {
+                const int v = src[ch];
+                dst[ch] = v;
+                if (v != 0) {
+                    first = min(first, ch * 32 + __ffs(v) - 1);
+                    last = ch * 32 + 31 - __clz(v);
                 }
             }
+            if (last >= 0) {
+                y0 = min(y0, ob0 + r);
+                y1 = ob0 + r;
+                x0 = min(x0, first);
+                x1 = max(x1, last);
+            }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-            y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-            x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-            x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        }
+        y0 = __reduce_min_sync(0xffffffffu, y0);
+        y1 = __reduce_max_sync(0xffffffffu, y1);
+        x0 = __reduce_min_sync(0xffffffffu, x0);
+        x1 = __reduce_max_sync(0xffffffffu, x1);
         if (lane == 0 && y1 >= 0) {
             atomicMin(&s_box[0], y0);
             atomicMax(&s_box[1], y1);
@@ -501,18 +499,20 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         if (threadIdx.x == 0) P.partials[part] = sat_box(T, ld, ob0, ob1, 0, P.Nx);
         return;
     }
-    // output box: x in 8-column strips [g_lo, g_hi], rows [yo_lo, yb_end) in 8-row groups
-    const int g_lo = max(0, x0 - K + 1) >> 3, g_hi = min(P.Nx - 1, x1) >> 3;
-    const int ns8 = g_hi - g_lo + 1, ns4 = 2 * ns8, sl0 = 2 * g_lo;
+    // output box: x in 12-column strips [0, ns12) from the float4 slot sl0 on, rows
+    // [yo_lo, yb_end) in 8-row groups
+    const int sl0 = max(0, x0 - K + 1) >> 2;
+    const int ns4 = (min(P.Nx - 1, x1) >> 2) - sl0 + 1;
+    const int ns12 = (ns4 + KB_XS / 4 - 1) / (KB_XS / 4);
     const int yo_lo = max(ob0, y0 - K + 1), yo_hi = min(ob1 - 1, y1);
     const int yb_end = min(ob1, yo_lo + 8 * ((yo_hi - yo_lo + 8) / 8));
-    const int xb0 = 8 * g_lo, xb_end = min(P.Nx, 8 * g_hi + 8);
+    const int xb0 = 4 * sl0, xb_end = min(P.Nx, xb0 + 4 * ns4);
     // the zero-model part, issued now so that its loads overlap the passes
     double outside = 0.0;
     if (threadIdx.x == 0)
         outside = sat_box(T, ld, ob0, ob1, 0, P.Nx) - sat_box(T, ld, yo_lo, yb_end, xb0, xb_end);
     // box-relative rows: float4 slots [sl0, sl0 + nsl), pitch bp (% 32 == 4)
-    const int nsl = 2 * (ns8 - 1) + NW;
+    const int nsl = KB_XS / 4 * (ns12 - 1) + NW;
     int bp = 4 * nsl;
     bp += ((4 - bp % 32) + 32) % 32;
     const int bp4 = bp / 4;
@@ -527,90 +527,85 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         const int rend = ys + 8 * ng + K - 1;                // rows [ys, rend) are read
         const int ly0 = max(y0, ys), ly1 = min(y1, rend - 1);
         if (P.counters && threadIdx.x == 0) {
-            if (ly0 <= ly1) c_x += (unsigned long long)(ly1 - ly0 + 1) * ns8 * 8 * K;
+            if (ly0 <= ly1) c_x += (unsigned long long)(ly1 - ly0 + 1) * ns12 * KB_XS * K;
             c_y += (unsigned long long)ng * ns4 * 32 * K;
             c_v += (unsigned long long)(ye - ys) * (xb_end - xb0);
         }
-        // load rows [ly0, ly1]: the 4-column groups that hold a nonzero value, zeros elsewhere
-        if (ly0 <= ly1) {
-            const int tc = min(nsl, NT), tr = NT / tc;
-            const int ti = threadIdx.x % tc, ty = threadIdx.x / tc;
-            if (ty < tr) {
-                for (int y = ly0 + ty; y <= ly1; y += tr) {
-                    const int* vrow = s_xr + (y - ob0) * P.nch;
-                    float4* d = reinterpret_cast<float4*>(S) + (y - ys) * bp4;
-                    const float4* g = src + (long long)y * (P.pitch / 4);
-                    for (int j = ti; j < nsl; j += tc) {
-                        // the slot's 4 columns hold a nonzero value: load them
-                        // (all written), else they are zeros
-                        const int sl = sl0 + j, ch = sl >> 3;
-                        const unsigned v = ch < P.nch ? (unsigned)vrow[ch] : 0u;
-                        if ((v >> (4 * (sl & 7))) & 0xfu)
-                            cp_async16(d + j, g + sl);
-                        else
-                            d[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                }
+        // load rows [ly0, ly1], a warp per row and a lane per float4 slot: the
+        // 4-column groups that hold a nonzero value (all written), zeros elsewhere
+        for (int j = lane; j < nsl; j += 32) {
+            const int sl = sl0 + j, ch = sl >> 3, sh = 4 * (sl & 7);
+            const bool in = ch < P.nch;
+            const int* m = s_xr + (ly0 + warp - ob0) * P.nch + (in ? ch : 0);
+            const float4* g = src + (long long)(ly0 + warp) * (P.pitch / 4) + (in ? sl : 0);
+            const long long gs = (long long)NWARPS * (P.pitch / 4);
+            float4* d = sm4 + (ly0 + warp - ys) * bp4 + j;
+#pragma unroll 4
+            for (int y = ly0 + warp; y <= ly1; y += NWARPS) {
+                cp_async16_or_zero(d, g, in && ((*m >> sh) & 0xf) != 0);
+                m += NWARPS * P.nch;
+                g += gs;
+                d += NWARPS * bp4;
             }
         }
-        // the other rows that the y FIR reads: zeros in its strips
+        // the other rows that the y FIR reads: zeros (whole rows, contiguous)
         {
-            const int tc = min(ns4, NT), tr = NT / tc;
-            const int ti = threadIdx.x % tc, ty = threadIdx.x / tc;
-            if (ty < tr) {
-                for (int y = ys + ty; y < rend; y += tr) {
-                    if (y >= ly0 && y <= ly1) continue;
-                    float4* d = reinterpret_cast<float4*>(S) + (y - ys) * bp4;
-                    for (int j = ti; j < ns4; j += tc) d[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int lo = ly0 <= ly1 ? (ly0 - ys) * bp4 : (rend - ys) * bp4;
+            for (int i = threadIdx.x; i < lo; i += NT) sm4[i] = z;
+            if (ly0 <= ly1)
+                for (int i = (ly1 + 1 - ys) * bp4 + threadIdx.x; i < (rend - ys) * bp4; i += NT)
+                    sm4[i] = z;
         }
         cp_async_wait_all();
         __syncthreads();
         // x FIR in place: S[y][xo] = sum_s vr[s] S[y][xo + s].  A warp owns whole
         // rows (ly0 + warp, + NWARPS, ...); its lanes take consecutive (row,
         // strip) pairs of those rows, 32 per pass.  Strip g writes columns
-        // [8g, 8g + 8) and reads columns >= 8g, so a row's strips in increasing
+        // [12 g, 12 g + 12) and reads columns >= 12 g, so a row's strips in increasing
         // order across passes, with loads before __syncwarp, never read a
-        // column that an earlier store of the row has overwritten.
+        // column that an earlier store of the row has overwritten.  Strips of
+        // 12: their float4 accesses lie 3 slots apart, which meets all banks
+        // (8-column strips were 2 apart, two-way conflicts).
         if (ly0 <= ly1) {
             float vr[K];
 #pragma unroll
             for (int s = 0; s < K; ++s) vr[s] = P.vr[s];
             const int nr = ly1 - ly0 + 1;
             const int nri = warp < nr ? (nr - 1 - warp) / NWARPS + 1 : 0;   // rows of this warp
-            const int npairs = nri * ns8;
-            const int di = 32 / ns8, dg = 32 % ns8;
-            int ri = lane / ns8, gi = lane % ns8;       // the lane's pair: row index, strip
+            const int npairs = nri * ns12;
+            const int di = 32 / ns12, dg = 32 % ns12;
+            int ri = lane / ns12, gi = lane % ns12;       // the lane's pair: row index, strip
             for (int q0 = 0; q0 < npairs; q0 += 32) {
                 const bool act = q0 + lane < npairs;
-                float4* row = reinterpret_cast<float4*>(S) + (ly0 + warp + NWARPS * ri - ys) * bp4;
+                float4* row = sm4 + (ly0 + warp + NWARPS * ri - ys) * bp4 + KB_XS / 4 * gi;
                 float w[4 * NW];
                 if (act) {
 #pragma unroll
                     for (int m = 0; m < NW; ++m) {
-                        const float4 f = row[2 * gi + m];
+                        const float4 f = row[m];
                         w[4 * m] = f.x; w[4 * m + 1] = f.y; w[4 * m + 2] = f.z; w[4 * m + 3] = f.w;
                     }
                 }
                 __syncwarp();
                 if (act) {
-                    float o[8];
+                    float o[KB_XS];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
+                    for (int q = 0; q < KB_XS; ++q) {
                         float acc = 0.f;
 #pragma unroll
                         for (int s = 0; s < K; ++s) acc += vr[s] * w[q + s];
                         o[q] = acc;
                     }
-                    row[2 * gi] = make_float4(o[0], o[1], o[2], o[3]);
-                    row[2 * gi + 1] = make_float4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+                    for (int q = 0; q < KB_XS; q += 4)
+                        row[q / 4] = make_float4(o[q], o[q + 1], o[q + 2], o[q + 3]);
                 }
                 __syncwarp();
                 ri += di;
                 gi += dg;
-                if (gi >= ns8) {
-                    gi -= ns8;
+                if (gi >= ns12) {
+                    gi -= ns12;
                     ++ri;
                 }
             }
@@ -701,18 +696,27 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
             }
             sum += s2.x + s2.y;
         } else {
-            // rows of any alignment: a warp per row, lanes along it
-            const int nw = xb_end - xb0;
-            for (int row = warp; row < ye - ys; row += NWARPS) {
-                const float* m = S + row * bp;
-                const int v0 = pbase + (ys + row) * P.Nx + xb0;
-                const float *od = P.obs + v0, *iw = P.iw + v0;
-                float* md = model ? model + (v0 - pbase) : nullptr;
-#pragma unroll 4
-                for (int x = lane; x < nw; x += 32) {
-                    const float r0 = (m[x] - od[x]) * iw[x];
-                    sum += r0 * r0;
-                    if (md) md[x] = m[x];
+            // rows of any alignment: flat index over the pass, stepped without
+            // divisions, several voxels in flight per thread
+            const int nw = xb_end - xb0, n = (ye - ys) * nw;
+            const int dq = NT / nw, dr = NT % nw;
+            const int row = threadIdx.x / nw;
+            int col = threadIdx.x % nw;
+            int si = row * bp + col, vi = pbase + (ys + row) * P.Nx + xb0 + col;
+            const int dsi = dq * bp + dr, dvi = dq * P.Nx + dr;
+#pragma unroll 8
+            for (int i = threadIdx.x; i < n; i += NT) {
+                const float m = S[si];
+                const float r0 = (m - P.obs[vi]) * P.iw[vi];
+                sum += r0 * r0;
+                if (model) model[vi - pbase] = m;
+                col += dr;
+                si += dsi;
+                vi += dvi;
+                if (col >= nw) {
+                    col -= nw;
+                    si += bp - nw;
+                    vi += P.Nx - nw;
                 }
             }
         }
