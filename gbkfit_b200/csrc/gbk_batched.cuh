@@ -381,6 +381,12 @@ __device__ __forceinline__ void cp_async16_or_zero(void* smem, const void* gmem,
                  : "memory");
 }
 
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
     int* const s_xr = reinterpret_cast<int*>(S + P.cap);        // (in1 - ob0, nch) range entries
     __shared__ float warp_part[NWARPS];
     __shared__ int s_box[4];
+    __shared__ double s_sat[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ld = P.Nx + 1;
     // blockIdx.x the set, blockIdx.y the (plane, band): sets vary fastest, so
@@ -507,10 +514,14 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
     const int yo_lo = max(ob0, y0 - K + 1), yo_hi = min(ob1 - 1, y1);
     const int yb_end = min(ob1, yo_lo + 8 * ((yo_hi - yo_lo + 8) / 8));
     const int xb0 = 4 * sl0, xb_end = min(P.Nx, xb0 + 4 * ns4);
-    // the zero-model part, issued now so that its loads overlap the passes
-    double outside = 0.0;
-    if (threadIdx.x == 0)
-        outside = sat_box(T, ld, ob0, ob1, 0, P.Nx) - sat_box(T, ld, yo_lo, yb_end, xb0, xb_end);
+    // the zero-model part: the corners of the band and of the box, copied to
+    // shared memory beside the rows (thread 0 sums them at the end)
+    if (threadIdx.x < 8) {
+        const bool outer = threadIdx.x < 4;
+        const int cy = threadIdx.x & 2 ? (outer ? ob1 : yb_end) : (outer ? ob0 : yo_lo);
+        const int cx = threadIdx.x & 1 ? (outer ? P.Nx : xb_end) : (outer ? 0 : xb0);
+        cp_async8(&s_sat[threadIdx.x], T + (long long)cy * ld + cx);
+    }
     // box-relative rows: float4 slots [sl0, sl0 + nsl), pitch bp (% 32 == 4)
     const int nsl = KB_XS / 4 * (ns12 - 1) + NW;
     int bp = 4 * nsl;
@@ -568,9 +579,6 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         // 12: their float4 accesses lie 3 slots apart, which meets all banks
         // (8-column strips were 2 apart, two-way conflicts).
         if (ly0 <= ly1) {
-            float vr[K];
-#pragma unroll
-            for (int s = 0; s < K; ++s) vr[s] = P.vr[s];
             const int nr = ly1 - ly0 + 1;
             const int nri = warp < nr ? (nr - 1 - warp) / NWARPS + 1 : 0;   // rows of this warp
             const int npairs = nri * ns12;
@@ -594,7 +602,7 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
                     for (int q = 0; q < KB_XS; ++q) {
                         float acc = 0.f;
 #pragma unroll
-                        for (int s = 0; s < K; ++s) acc += vr[s] * w[q + s];
+                        for (int s = 0; s < K; ++s) acc += P.vr[s] * w[q + s];
                         o[q] = acc;
                     }
 #pragma unroll
@@ -614,7 +622,7 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         // y FIR in place: model(yo, xo) = sum_t ur[t] S[yo + t][xo], written to S row yo.
         // Packed FP32 pairs (FFMA2: two lanes of fma, each rounded as fmaf),
         // columns (x, x+1) and (x+2, x+3) of a float4 per instruction.  Items
-        // (8-row group, float4 column) in ascending order, NT per round, loads
+        // (row group, float4 column) in ascending order, NT per round, loads
         // before the round's barrier and stores after it: a column's group is
         // written only after every lower group of that column, the only
         // readers of its rows, has loaded them.
@@ -731,6 +739,9 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
     if (threadIdx.x == 0) {
         float s = 0.f;
         for (int w = 0; w < NWARPS; ++w) s += warp_part[w];
+        // corners [y1][x1] - [y0][x1] - [y1][x0] + [y0][x0], band minus box
+        const double outside = (s_sat[3] - s_sat[1] - s_sat[2] + s_sat[0]) -
+                               (s_sat[7] - s_sat[5] - s_sat[6] + s_sat[4]);
         P.partials[part] = (double)s + outside;
         if (P.counters) {
             atomicAdd(&P.counters[GBK_CTR_KB_XFMA], c_x);
