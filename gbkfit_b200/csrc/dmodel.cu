@@ -6,29 +6,41 @@
 // gbkfit_host/include/gbkfit/host/kernels.hpp:55-135, 484-514.
 #include "gbk_common.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace gbk {
 
-// dmodels.hpp:7-46: box average of scale-sized blocks starting at offset
-__global__ void downscale_kernel(int scx, int scy, int scz, int ofx, int ofy, int ofz, int srx,
-                                 int sry, int dsx, int dsy, int dsz, const float* src, float* dst)
+// dmodels.hpp:7-46: box average of scale-sized blocks starting at offset.
+// Block (32, 8): lanes along x, rows of y; a thread takes four z, whose loads
+// are independent.  Bound by memory: 256 x 256 x 128 cropped from 320 x 320 x
+// 160 in 29 us, 46 us with a 64-bit index division per voxel.
+constexpr int DS_Z = 4;
+__global__ void __launch_bounds__(256) downscale_kernel(int scx, int scy, int scz, int ofx,
+                                                        int ofy, int ofz, int srx, int sry,
+                                                        int dsx, int dsy, int dsz,
+                                                        const float* __restrict__ src,
+                                                        float* __restrict__ dst)
 {
     const float nf = 1.0f / (scx * scy * scz);
-    long long n = (long long)dsx * dsy * dsz;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int x = (int)(i % dsx);
-        int y = (int)((i / dsx) % dsy);
-        int z = (int)(i / ((long long)dsx * dsy));
-        int nx = ofx + x * scx, ny = ofy + y * scy, nz = ofz + z * scz;
-        float sum = 0;
-        for (int dz = 0; dz < scz; ++dz)
-            for (int dy = 0; dy < scy; ++dy)
-                for (int dx = 0; dx < scx; ++dx)
-                    sum += src[idx3(nx + dx, ny + dy, nz + dz, srx, sry)];
-        dst[i] = sum * nf;
-    }
+    const int x = blockIdx.x * 32 + threadIdx.x;
+    if (x >= dsx) return;
+    for (int y = blockIdx.y * 8 + threadIdx.y; y < dsy; y += 8 * gridDim.y)
+        for (int z0 = blockIdx.z * DS_Z; z0 < dsz; z0 += DS_Z * gridDim.z) {
+            float sum[DS_Z] = {};
+            const float* s0 = src + idx3(ofx + x * scx, ofy + y * scy, ofz + z0 * scz, srx, sry);
+            const long long plane = (long long)srx * sry;
+            for (int dz = 0; dz < scz; ++dz)
+                for (int dy = 0; dy < scy; ++dy)
+                    for (int dx = 0; dx < scx; ++dx)
+#pragma unroll
+                        for (int k = 0; k < DS_Z; ++k)
+                            if (z0 + k < dsz)
+                                sum[k] += s0[dx + (long long)dy * srx + (k * scz + dz) * plane];
+#pragma unroll
+            for (int k = 0; k < DS_Z; ++k)
+                if (z0 + k < dsz) dst[idx3(x, y, z0 + k, dsx, dsy)] = sum[k] * nf;
+        }
 }
 
 // dmodels.hpp:48-74
@@ -58,6 +70,11 @@ __global__ void mask_kernel(float cutoff, int apply, long long n, float* d, floa
 // * orders >= 3 take a second pass over the column with (v - m1)^k in fp64,
 //   without dz, divided by m0, as the reference does.
 // mm receives the mask map, mw the weight map.
+// Bound by the latency of a column walked in order (the fp32 sum): thirty-two
+// channels are loaded at once, and blocks are one warp, so that small maps
+// spread over the chip (64 x 64 x 64: 7.0 us, 8.1 us with four at a time and
+// 128 threads a block).
+constexpr int MOM_Z = 32;
 __global__ void moments_kernel(int nx, int ny, int nz, float stz, float zz, const float* d,
                                const float* w, float cutoff, int norders, const int* orders,
                                float* md, float* mm, float* mw)
@@ -71,17 +88,26 @@ __global__ void moments_kernel(int nx, int ny, int nz, float stz, float zz, cons
     double s0 = 0, s1 = 0, s2 = 0, sw = 0;
     const float* dp = d + i2;
     const float* wp = w ? w + i2 : nullptr;
-#pragma unroll 4
-    for (int z = 0; z < nz; ++z) {
-        const float dv = dp[sxy * z];
-        const float ddz = dv * stz;
-        m0s += ddz;
-        const double v = (double)(zz + z * stz);
-        const double a = (double)ddz;
-        s0 += a;
-        s1 += a * v;
-        s2 += a * v * v;
-        if (wp) sw += (double)wp[sxy * z] * a;
+    for (int z0 = 0; z0 < nz; z0 += MOM_Z) {
+        float dv[MOM_Z], wv[MOM_Z];
+#pragma unroll
+        for (int k = 0; k < MOM_Z; ++k) {
+            const bool in = z0 + k < nz;
+            dv[k] = in ? dp[sxy * (z0 + k)] : 0.f;
+            wv[k] = in && wp ? wp[sxy * (z0 + k)] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < MOM_Z; ++k) {
+            if (z0 + k >= nz) break;
+            const float ddz = dv[k] * stz;
+            m0s += ddz;
+            const double v = (double)(zz + (z0 + k) * stz);
+            const double a = (double)ddz;
+            s0 += a;
+            s1 += a * v;
+            s2 += a * v * v;
+            if (wp) sw += (double)wv[k] * a;
+        }
     }
     const bool valid = fabsf(m0s) > cutoff;
     mm[i2] = valid ? 1.f : 0.f;
@@ -170,13 +196,17 @@ __global__ void __launch_bounds__(SUM_THREADS) residual_sum_partial(const float*
     }
 }
 
-__global__ void residual_sum_final(const double* part, int nparts, float* out)
+// one warp: lane-strided fp64 sums, then a fixed shuffle tree (a serial loop
+// over the 296 partials took 7.9 us, this 3.3)
+__global__ void __launch_bounds__(32) residual_sum_final(const double* part, int nparts,
+                                                         float* out)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0;
-        for (int i = 0; i < nparts; ++i) s += part[i];
-        out[0] = (float)s;
-    }
+    double s = 0;
+#pragma unroll 10
+    for (int i = threadIdx.x; i < nparts; i += 32) s += part[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[0] = (float)s;
 }
 
 static int grid_for(long long n, int threads)
@@ -203,7 +233,9 @@ extern "C" int gbkb200_dmodel_dcube_downscale_f32(gbkb200_ctx* ctx, const int sc
     }
     long long n = (long long)dst_size[0] * dst_size[1] * dst_size[2];
     if (n == 0) return gbk_finish(ctx);
-    downscale_kernel<<<grid_for(n, 256), 256, 0, ctx->stream>>>(
+    const dim3 grid((dst_size[0] + 31) / 32, std::min((dst_size[1] + 7) / 8, 65535),
+                    std::min((dst_size[2] + DS_Z - 1) / DS_Z, 65535));
+    downscale_kernel<<<grid, dim3(32, 8), 0, ctx->stream>>>(
         scale[0], scale[1], scale[2], offset[0], offset[1], offset[2], src_size[0], src_size[1],
         dst_size[0], dst_size[1], dst_size[2], src, dst);
     GBK_CUDA_TRY(cudaGetLastError());
@@ -238,8 +270,8 @@ extern "C" int gbkb200_dmodel_mmaps_moments_f32(gbkb200_ctx* ctx, const int size
     float* wmap = mmaps_m;
     if (!mask || (dcube_w && !wmap)) return GBKB200_ERR_INVALID_ARG;
     if (size[0] < 1 || size[1] < 1 || size[2] < 1) return GBKB200_ERR_INVALID_ARG;
-    dim3 grid((size[0] + 127) / 128, size[1]);
-    moments_kernel<<<grid, 128, 0, ctx->stream>>>(size[0], size[1], size[2], step[2], zero[2],
+    dim3 grid((size[0] + 31) / 32, size[1]);
+    moments_kernel<<<grid, 32, 0, ctx->stream>>>(size[0], size[1], size[2], step[2], zero[2],
                                                   dcube_d, dcube_w, cutoff, norders, orders,
                                                   mmaps_d, mask, wmap);
     GBK_CUDA_TRY(cudaGetLastError());
