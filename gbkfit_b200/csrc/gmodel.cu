@@ -11,8 +11,8 @@
 //    coalesced 128-byte row update; each voxel has a single writer, so the
 //    accumulation needs no atomics;
 //  * thick disks: a block owns a 32-spaxel row segment, its warps walk the
-//    spatial z axis and accumulate the spectral columns in shared memory
-//    (shared atomics), then add each column to HBM once;
+//    spatial z axis and accumulate the spectral columns in shared memory (one
+//    owner per channel), then add each column to HBM once;
 //  * mcdisk: one thread per cloud, Philox counter-based random numbers keyed by
 //    (seed, cloud), red.global.add into the cube (mode 0) or an ordered
 //    two-pass fixed-point accumulation (mode 1, deterministic).
@@ -22,12 +22,16 @@
 
 namespace gbk {
 
-// Thin disk: one thread per spaxel (spatial z = 1).  Block (32, 8): a warp is
-// a run of 32 adjacent x at one y.
-__global__ void __launch_bounds__(256) smdisk_thin_kernel(DiskArgs a, int* status)
+// Thin disk: one thread per spaxel (spatial z = 1).  Block (32, 2): a warp is
+// a run of 32 adjacent x at one y.  Bound by latency: the channels of a column
+// are read eight at a time before any is written back (one at a time, each read
+// waited for the write before it), and blocks are two warps so that a small
+// plane spreads over the chip (96 x 96 x 96: 14 us, 21 us before).
+constexpr int THIN_Y = 2, THIN_Z = 8;
+__global__ void __launch_bounds__(32 * THIN_Y) smdisk_thin_kernel(DiskArgs a, int* status)
 {
     const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * 8 + threadIdx.y;
+    const int y = blockIdx.y * THIN_Y + threadIdx.y;
     const bool inside = x < a.sx && y < a.sy;
     int bad = 0;
     DiskConst kc = disk_const(a);
@@ -53,72 +57,28 @@ __global__ void __launch_bounds__(256) smdisk_thin_kernel(DiskArgs a, int* statu
     if (a.scube) {
         const long long plane = (long long)a.sx * a.sy;
         float* col = a.scube + (x + (long long)a.sx * y);
-        for (int z = wlo; z <= whi; ++z) {
-            if (z >= zlo && z <= zhi) {
-                float zv = a.spec_zero + z * a.spec_step;
-                float d = zv - o.vv;
-                col[plane * z] += o.orv * (amp * expf(-d * d / inv2c2));
+        for (int z0 = wlo; z0 <= whi; z0 += THIN_Z) {
+            float c[THIN_Z];
+#pragma unroll
+            for (int k = 0; k < THIN_Z; ++k) {
+                const int z = z0 + k;
+                c[k] = z >= zlo && z <= zhi ? col[plane * z] : 0.f;
             }
-        }
-    }
-    if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
-}
-
-// Thick disk (or thin with spatial z > 1): block (32, 8) owns 32 adjacent
-// spaxel columns of one row; each warp takes every 8th spatial z and adds its
-// lines into a shared (spec_size x 32) column tile; the tile is then added to
-// the cube.  With USE_SMEM = false (spectra too long for shared memory) the
-// lines go straight to HBM with atomics.
-template<bool USE_SMEM>
-__global__ void __launch_bounds__(256) smdisk_thick_kernel(DiskArgs a, int* status)
-{
-    extern __shared__ float tile[];
-    const int tx = threadIdx.x, tz = threadIdx.y;
-    const int x = blockIdx.x * 32 + tx;
-    const int y = blockIdx.y;
-    const long long plane = (long long)a.sx * a.sy;
-    int bad = 0;
-    if (USE_SMEM && a.scube) {
-        for (int i = tz * 32 + tx; i < a.spec_size * 32; i += 256) tile[i] = 0.f;
-        __syncthreads();
-    }
-    DiskConst kc = disk_const(a);
-    if (x < a.sx) {
-        for (int z = tz; z < a.sz; z += 8) {
-            SpaxelOut o;
-            if (!smdisk_spaxel(a, kc, x, y, z, o, bad)) continue;
-            if (a.image) atomicAdd(&a.image[x + (long long)a.sx * y], o.orv);
-            smdisk_side_outputs(a, x, y, z, o);
-            int zlo, zhi;
-            if (a.scube && line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
-                float amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
-                float inv2c2 = 2 * o.dv * o.dv;
-                for (int zs = zlo; zs <= zhi; ++zs) {
-                    float zv = a.spec_zero + zs * a.spec_step;
+#pragma unroll
+            for (int k = 0; k < THIN_Z; ++k) {
+                const int z = z0 + k;
+                if (z >= zlo && z <= zhi) {
+                    float zv = a.spec_zero + z * a.spec_step;
                     float d = zv - o.vv;
-                    float f = o.orv * (amp * expf(-d * d / inv2c2));
-                    if (USE_SMEM) atomicAdd(&tile[zs * 32 + tx], f);
-                    else atomicAdd(&a.scube[x + (long long)a.sx * y + plane * zs], f);
+                    col[plane * z] = c[k] + o.orv * (amp * expf(-d * d / inv2c2));
                 }
             }
         }
     }
-    if (USE_SMEM && a.scube) {
-        __syncthreads();
-        if (x < a.sx) {
-            float* col = a.scube + (x + (long long)a.sx * y);
-            for (int zs = tz; zs < a.spec_size; zs += 8) {
-                float v = tile[zs * 32 + tx];
-                if (v != 0.f) col[plane * zs] += v;
-            }
-        }
-    }
     if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
 }
 
-// ---- mcdisk ------------------------------------------------------------------
-
-// The cloud's line at distance d from its centre without the amplitude:
+// A line at distance d from its centre without the amplitude:
 // exp(-d^2 / (2 sigma^2)) as 2^(-d^2 rinv) with rinv = log2(e) / (2 sigma^2),
 // by the PTX ex2.approx instruction (relative error ~2^-22; inside the +-5
 // sigma window the argument is >= -18.1, far from the flush to zero)
@@ -128,6 +88,80 @@ __device__ __forceinline__ float line_e2(float d, float rinv)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-(d * d) * rinv));
     return e;
 }
+
+// Thick disk (or thin with spatial z > 1): block (32, 16) owns 32 adjacent
+// spaxel columns of one row.  Its warps evaluate sixteen spatial z at a time and
+// put their lines' parameters into shared memory; then warp w adds, for every
+// line of the round, the channels w, w + 16, ... of the columns, each channel of
+// a column having one owner: no atomics, and sums in a fixed order (shared
+// fp32 atomics took 145 us for a 96 x 96 x 96 grid with 96 channels, this 59).
+// With USE_SMEM the spectral columns (spec_size x 32) are accumulated in shared
+// memory and added to the cube at the end; else (spectra too long) in the cube.
+constexpr int TH = 16;          // warps: a power of two
+template<bool USE_SMEM>
+__global__ void __launch_bounds__(32 * TH) smdisk_thick_kernel(DiskArgs a, int* status)
+{
+    extern __shared__ float tile[];
+    __shared__ float s_v[TH][32], s_amp[TH][32], s_rinv[TH][32];
+    __shared__ int s_lo[TH][32], s_hi[TH][32];
+    const int tx = threadIdx.x, tz = threadIdx.y;
+    const int x = blockIdx.x * 32 + tx;
+    const int y = blockIdx.y;
+    const long long plane = (long long)a.sx * a.sy;
+    int bad = 0;
+    if (USE_SMEM && a.scube)
+        for (int i = tz * 32 + tx; i < a.spec_size * 32; i += 32 * TH) tile[i] = 0.f;
+    DiskConst kc = disk_const(a);
+    float* col = a.scube ? a.scube + (x + (long long)a.sx * y) : nullptr;
+    for (int z0 = 0; z0 < a.sz; z0 += TH) {
+        const int z = z0 + tz;
+        SpaxelOut o;
+        int zlo = 0, zhi = -1;
+        float amp = 0.f, rinv = 0.f, v = 0.f;
+        if (x < a.sx && z < a.sz && smdisk_spaxel(a, kc, x, y, z, o, bad)) {
+            if (a.image) atomicAdd(&a.image[x + (long long)a.sx * y], o.orv);
+            smdisk_side_outputs(a, x, y, z, o);
+            if (a.scube &&
+                line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
+                amp = o.orv * (1 / (o.dv * sqrtf(2 * GBK_PI)));
+                rinv = 0.7213475204444817f / (o.dv * o.dv);
+                v = o.vv;
+            } else {
+                zlo = 0;
+                zhi = -1;
+            }
+        }
+        if (!a.scube) continue;             // every thread
+        s_v[tz][tx] = v;
+        s_amp[tz][tx] = amp;
+        s_rinv[tz][tx] = rinv;
+        s_lo[tz][tx] = zlo;
+        s_hi[tz][tx] = zhi;
+        __syncthreads();
+        for (int k = 0; k < TH; ++k) {
+            const int lo = s_lo[k][tx], hi = s_hi[k][tx];
+            const float vk = s_v[k][tx], ak = s_amp[k][tx], ik = s_rinv[k][tx];
+            // the first channel >= lo that is tz modulo TH
+            for (int zs = lo + ((tz - lo) & (TH - 1)); zs <= hi; zs += TH) {
+                const float d = (a.spec_zero + zs * a.spec_step) - vk;
+                const float f = ak * line_e2(d, ik);
+                if (USE_SMEM) tile[zs * 32 + tx] += f;
+                else col[plane * zs] += f;
+            }
+        }
+        __syncthreads();
+    }
+    if (USE_SMEM && a.scube && x < a.sx) {
+        // the channels this thread owns
+        for (int zs = tz; zs < a.spec_size; zs += TH) {
+            const float f = tile[zs * 32 + tx];
+            if (f != 0.f) col[plane * zs] += f;
+        }
+    }
+    if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
+}
+
+// ---- mcdisk ------------------------------------------------------------------
 
 // Philox-4x32-10 (Salmon et al., SC'11), counter {ci, k/4, 0, 0}, key = seed
 struct Philox {
@@ -494,32 +528,50 @@ __global__ void __launch_bounds__(256) mcdisk_v4_kernel(DiskArgs a, McArgs m, fl
 }
 
 // scube[z][s] += sum over the copies c of lines[c][s][z] (in copy order) for
-// spaxels s < nsp, channels z < nz (32 x 32 tiles)
+// spaxels s < nsp, channels z < nz.  Tiles of 64 spaxels x 32 channels: the
+// scratch is read in 16-byte pieces along z and the cube's values are requested
+// before the tile is complete, so that a thread keeps ten loads in flight.
+// Bound by HBM: 320 x 320 x 160 49 us (92 us with 32 x 32 tiles of 4-byte
+// loads).
 __global__ void __launch_bounds__(256) mc_lines_add_kernel(const float* __restrict__ lines,
                                                            float* __restrict__ scube,
                                                            long long nsp, int nzp, int nz,
                                                            int copies)
 {
-    __shared__ float tile[32][33];
-    const long long s0 = (long long)blockIdx.x * 32;
+    __shared__ float tile[32][65];
+    const long long s0 = (long long)blockIdx.x * 64;
     const int z0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const long long cstride = nsp * nzp;
+    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+    float old[8];
 #pragma unroll
-    for (int k = 0; k < 32; k += 8) {
-        const long long s = s0 + ty + k;
-        const int z = z0 + tx;
-        float v = 0.f;
-        if (s < nsp && z < nz)
-            for (int c = 0; c < copies; ++c) v += lines[c * cstride + s * nzp + z];
-        tile[ty + k][tx] = v;
+    for (int k = 0; k < 8; ++k) {
+        const int z = z0 + ty + 4 * k;
+        old[k] = s0 + tx < nsp && z < nz ? scube[(long long)z * nsp + s0 + tx] : 0.f;
+    }
+    // 8 pieces of 4 channels per spaxel (nzp is a multiple of 4)
+    const int q = threadIdx.x & 7, r = threadIdx.x >> 3;
+#pragma unroll
+    for (int h = 0; h < 64; h += 32) {
+        const long long s = s0 + r + h;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s < nsp && z0 + 4 * q < nzp)
+            for (int c = 0; c < copies; ++c) {
+                const float4 t =
+                    *reinterpret_cast<const float4*>(lines + c * cstride + s * nzp + z0 + 4 * q);
+                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+            }
+        tile[4 * q][r + h] = v.x;
+        tile[4 * q + 1][r + h] = v.y;
+        tile[4 * q + 2][r + h] = v.z;
+        tile[4 * q + 3][r + h] = v.w;
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 32; k += 8) {
-        const int z = z0 + ty + k;
-        const long long s = s0 + tx;
-        if (s < nsp && z < nz) scube[(long long)z * nsp + s] += tile[tx][ty + k];
+    for (int k = 0; k < 8; ++k) {
+        const int zl = ty + 4 * k;
+        if (s0 + tx < nsp && z0 + zl < nz)
+            scube[(long long)(z0 + zl) * nsp + s0 + tx] = old[k] + tile[zl][tx];
     }
 }
 
@@ -720,10 +772,10 @@ int gbk_launch_smdisk(const DiskArgs& a, cudaStream_t stream, int* status)
 {
     const bool thin = a.rht.uids == nullptr;
     if (thin && a.sz == 1) {
-        dim3 block(32, 8), grid((a.sx + 31) / 32, (a.sy + 7) / 8);
+        dim3 block(32, THIN_Y), grid((a.sx + 31) / 32, (a.sy + THIN_Y - 1) / THIN_Y);
         smdisk_thin_kernel<<<grid, block, 0, stream>>>(a, status);
     } else {
-        dim3 block(32, 8), grid((a.sx + 31) / 32, a.sy);
+        dim3 block(32, TH), grid((a.sx + 31) / 32, a.sy);
         size_t smem = a.scube ? (size_t)a.spec_size * 32 * sizeof(float) : 0;
         if (smem <= 200 * 1024) {
             const int rc = gbk_raise_smem_limit(
@@ -809,7 +861,7 @@ extern "C" int gbkb200_gmodel_mcdisk_evaluate_f32(gbkb200_ctx* ctx, float cflux,
         GBK_CUDA_TRY(cudaMemsetAsync(lines, 0, need, ctx->stream));
         mcdisk_v4_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, lines, nzp, copies,
                                                           ctx->d_status);
-        const dim3 tg((unsigned)((nsp + 31) / 32), (unsigned)((a.spec_size + 31) / 32));
+        const dim3 tg((unsigned)((nsp + 63) / 64), (unsigned)((a.spec_size + 31) / 32));
         mc_lines_add_kernel<<<tg, 256, 0, ctx->stream>>>(lines, a.scube, nsp, nzp, a.spec_size,
                                                          copies);
         GBK_CUDA_TRY(cudaGetLastError());
