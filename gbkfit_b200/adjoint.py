@@ -147,14 +147,16 @@ class SMDiskChi2:
         self.pcube = f32(pc)
         # adjoint of the circular convolution: convolution with k(-i mod P)
         self.pcube_adj = f32(np.roll(pc[::-1, ::-1, ::-1], 1, axis=(0, 1, 2)))
-        self.out2 = torch.zeros(2, dtype=torch.float64, device=self.dev)
         self.nsub = len(disk.subrnodes)
-        self.gsub = torch.zeros(3 * self.nsub + 5, dtype=torch.float64, device=self.dev)
+        # chi^2 and its scale derivative, then the sub-node gradient: one copy back
+        self._out = torch.zeros(2 + 3 * self.nsub + 5, dtype=torch.float64, device=self.dev)
+        self._out_h = torch.empty(self._out.shape, dtype=torch.float64, pin_memory=True)
+        self.out2, self.gsub = self._out[:2], self._out[2:]
         self.jac = interpolation_jacobian(disk)
         self.names = param_names(disk)
         self.nnodes = len(disk.rnodes)
         self._theta = None
-        self._keep = None
+        self._keep, self._views = self._alloc_disk()
 
     # ---- parameters ----------------------------------------------------------
     def params(self, theta):
@@ -166,19 +168,41 @@ class SMDiskChi2:
         return to_vector(params, scale)
 
     # ---- passes --------------------------------------------------------------
+    def _alloc_disk(self):
+        """The disk's device arrays: the trait tables once, and the arrays that
+        depend on the parameters as views of one buffer, filled by one copy from
+        one pinned buffer per evaluation ({name or kind: its host view})."""
+        up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(self.dev)
+        d = self.disk
+        sizes = [(n, d.common_size(n)) for n in GEOMETRY if n in d.pdescs]
+        sizes += [(k, max(d.tables[k]['npv'], 1)) for k in KINDS if d.tables[k] is not None]
+        total = sum(n for _, n in sizes)
+        self._flat_d = torch.zeros(total, dtype=torch.float32, device=self.dev)
+        self._flat_h = torch.zeros(total, dtype=torch.float32, pin_memory=True)
+        dev, host, off = {n: None for n in GEOMETRY + KINDS}, {}, 0
+        dev['subrnodes'] = up(d.subrnodes.astype(np.float32))
+        for name, n in sizes:
+            dv, host[name] = self._flat_d[off:off + n], self._flat_h[off:off + n].numpy()
+            off += n
+            if name in GEOMETRY:
+                dev[name] = dv
+            else:
+                t = d.tables[name]
+                dev[name] = dict({f: up(t[f]) for f in ('uids', 'cvalues', 'ccounts', 'pcounts')},
+                                 pvalues=dv)
+        return dev, host
+
     def _forward(self, theta):
         p, scale = self.params(theta)
         packed = self.disk.pack(p)
-        dev = {}
-        for k, v in packed.items():
-            if v is None:
-                dev[k] = None
-            elif isinstance(v, dict):
-                dev[k] = {f: torch.from_numpy(np.ascontiguousarray(a)).to(self.dev)
-                          for f, a in v.items()}
-            else:
-                dev[k] = torch.from_numpy(np.ascontiguousarray(v)).to(self.dev)
-        self._keep = dev
+        # every public call waits for the stream: the pinned buffer is free again
+        for name, h in self._views.items():
+            v = packed[name]
+            v = v['pvalues'] if isinstance(v, dict) else v
+            h[:v.size] = v
+        dev = self._keep
+        with torch.cuda.stream(self.stream):
+            self._flat_d.copy_(self._flat_h, non_blocking=True)
         tr = {k: ((dev[k]['uids'], dev[k]['cvalues'], dev[k]['ccounts'], dev[k]['pvalues'],
                    dev[k]['pcounts']) if dev[k] is not None else (None,) * 5) for k in KINDS}
         ss, st, sz = self.geom.spat()
@@ -225,6 +249,14 @@ class SMDiskChi2:
     def _assemble(self, out2, gsub):
         return assemble_gradient(self.jac, gsub, out2[1])
 
+    def _results(self):
+        """(out2, gsub) on the host (synchronises)."""
+        with torch.cuda.stream(self.stream):
+            self._out_h.copy_(self._out, non_blocking=True)
+        self.stream.synchronize()
+        out = self._out_h.numpy().copy()
+        return out[:2], out[2:]
+
     # ---- public --------------------------------------------------------------
     def value(self, theta):
         """chi^2 at theta (synchronises)."""
@@ -236,9 +268,8 @@ class SMDiskChi2:
         """(chi^2, d chi^2 / d theta) at theta (synchronises)."""
         self._forward(theta)
         self._backward()
-        self.stream.synchronize()
-        out2 = self.out2.cpu().numpy()
-        return float(out2[0]), self._assemble(out2, self.gsub.cpu().numpy())
+        out2, gsub = self._results()
+        return float(out2[0]), self._assemble(out2, gsub)
 
     def grad_after_forward(self, theta):
         """The gradient at theta, reusing the residual adjoint of the last
@@ -247,9 +278,7 @@ class SMDiskChi2:
         if self._theta is None or not np.array_equal(th, self._theta):
             self._forward(th)
         self._backward()
-        self.stream.synchronize()
-        out2 = self.out2.cpu().numpy()
-        return self._assemble(out2, self.gsub.cpu().numpy())
+        return self._assemble(*self._results())
 
 
 class SMDiskChi2Function(torch.autograd.Function):

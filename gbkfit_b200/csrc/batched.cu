@@ -411,7 +411,7 @@ static void launch_ka(const gbkb200_batch* bt, const BatchKernelArgs& P, int cn,
                            ? (P.Wy + 3) / 4 * P.nch
                            : (P.Wy * P.nch + KA_THREADS / 32 - 1) / (KA_THREADS / 32);
     const size_t smem = bt->ka_tiles ? (size_t)P.Nz * 16 : 0;
-    bt->ka<<<dim3(blocks, cn), KA_THREADS, smem, st>>>(P, bt->ctx->d_status);
+    bt->ka<<<dim3(blocks, cn), KA_THREADS, smem, st>>>(P, gbk_status(bt->ctx));
 }
 
 static KaFn ka_fn(int Kz)
@@ -1074,7 +1074,7 @@ extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float*
         const int cn = std::min(bt->chunk, nsets - s0);
         P.set0 = s0;
         stage_mark(bt, 0, true);
-        k1_model_xfft<<<dim3(P.Wy, cn), 512, bt->smem1, st>>>(P, bt->ctx->d_status);
+        k1_model_xfft<<<dim3(P.Wy, cn), 512, bt->smem1, st>>>(P, gbk_status(bt->ctx));
         stage_mark(bt, 0, false);
         stage_mark(bt, 1, true);
         // K2: y forward over (z < Wz, kx); columns stride hx, outer stride Py * hx

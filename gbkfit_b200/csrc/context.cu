@@ -11,6 +11,23 @@ static thread_local cudaError_t g_last_cuda_error = cudaSuccess;
 
 void gbk_set_last_cuda_error(cudaError_t e) { g_last_cuda_error = e; }
 
+static int status_code(int s)
+{
+    if (!s) return GBKB200_OK;
+    if (s & GBK_STATUS_BAD_TRAIT) return GBKB200_ERR_BAD_TRAIT;
+    if (s & GBK_STATUS_TIMEOUT) return GBKB200_ERR_TIMEOUT;
+    return GBKB200_ERR_INVALID_ARG;
+}
+
+// reads and clears the mapped word (the stream has been waited for)
+static int take_mapped_status(gbkb200_ctx* ctx)
+{
+    volatile int* w = ctx->h_status + 1;
+    const int s = *w;
+    if (s) *w = 0;
+    return status_code(s);
+}
+
 int gbk_finish(gbkb200_ctx* ctx)
 {
     cudaError_t e = cudaGetLastError();
@@ -19,7 +36,10 @@ int gbk_finish(gbkb200_ctx* ctx)
         return GBKB200_ERR_CUDA;
     }
     if (!ctx->sync) return GBKB200_OK;
-    return gbkb200_ctx_synchronize(ctx);
+    // the first wait after asynchronous calls reads the device's word as well
+    if (ctx->async_calls) return gbkb200_ctx_synchronize(ctx);
+    GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    return take_mapped_status(ctx);
 }
 
 extern "C" int gbkb200_ctx_create(gbkb200_ctx** out, int device)
@@ -31,12 +51,12 @@ extern "C" int gbkb200_ctx_create(gbkb200_ctx** out, int device)
     if (!c) return GBKB200_ERR_OOM;
     c->device = device;
     if (cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&c->h_status, sizeof(int)) != cudaSuccess) {
+        cudaMallocHost(&c->h_status, 2 * sizeof(int)) != cudaSuccess) {
         if (c->d_status) cudaFree(c->d_status);
         delete c;
         return GBKB200_ERR_OOM;
     }
-    *c->h_status = 0;
+    c->h_status[0] = c->h_status[1] = 0;
     GBK_CUDA_TRY(cudaMemset(c->d_status, 0, sizeof(int)));
     *out = c;
     return GBKB200_OK;
@@ -67,6 +87,7 @@ extern "C" int gbkb200_ctx_set_sync(gbkb200_ctx* ctx, int sync)
 {
     if (!ctx) return GBKB200_ERR_INVALID_ARG;
     ctx->sync = sync ? 1 : 0;
+    if (!ctx->sync) ctx->async_calls = 1;
     return GBKB200_OK;
 }
 
@@ -108,16 +129,15 @@ extern "C" int gbkb200_ctx_synchronize(gbkb200_ctx* ctx)
     GBK_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
     GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (ctx->sync) ctx->async_calls = 0;
     int s = *ctx->h_status;
     if (s) {
         GBK_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
         GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         *ctx->h_status = 0;
-        if (s & GBK_STATUS_BAD_TRAIT) return GBKB200_ERR_BAD_TRAIT;
-        if (s & GBK_STATUS_TIMEOUT) return GBKB200_ERR_TIMEOUT;
-        return GBKB200_ERR_INVALID_ARG;
+        return status_code(s);
     }
-    return GBKB200_OK;
+    return take_mapped_status(ctx);
 }
 
 extern "C" const char* gbkb200_error_string(int code)

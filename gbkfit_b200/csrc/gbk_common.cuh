@@ -70,11 +70,12 @@ struct gbkb200_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     int sync = 1;
+    int async_calls = 0;          // calls may have been made in asynchronous mode
     unsigned long long seed = 42;
     int mc_mode = 0;
     int fft_mode = 0;             // 1: mixed-radix passes only (gbkb200_ctx_set_fft)
     int* d_status = nullptr;      // device status word (GBK_STATUS_* bits)
-    int* h_status = nullptr;      // pinned mirror
+    int* h_status = nullptr;      // pinned: its mirror, and the mapped word below
     void* fft_state = nullptr;    // FFT plan / spectrum caches (fft.cu)
     void* reduce_scratch = nullptr;
     size_t reduce_scratch_bytes = 0;
@@ -83,6 +84,13 @@ struct gbkb200_ctx {
     void* serve_scratch = nullptr;  // block partials + last-block counter (serve.cu)
 };
 
+// The status word that a call's kernels write: the device's, which asynchronous
+// callers copy on their stream, or in sync mode a mapped pinned one, which the
+// host reads after its wait (a 4-byte copy per call cost 5-8 us beside it).
+inline int* gbk_status(const gbkb200_ctx* ctx)
+{
+    return ctx->sync ? ctx->h_status + 1 : ctx->d_status;
+}
 int gbk_finish(gbkb200_ctx* ctx);   // launch check, and sync + status read in sync mode
 // Raises kernel fn's dynamic shared-memory limit on the current device to at
 // least `bytes`, never lowering it: the limit is one setting per function,

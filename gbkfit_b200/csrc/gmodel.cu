@@ -797,7 +797,7 @@ extern "C" int gbkb200_gmodel_smdisk_evaluate_f32(gbkb200_ctx* ctx, GBKB200_DISK
     GBK_FILL_DISK(a);
     int rc = check_disk(a);
     if (rc) return rc;
-    rc = gbk_launch_smdisk(a, ctx->stream, ctx->d_status);
+    rc = gbk_launch_smdisk(a, ctx->stream, gbk_status(ctx));
     if (rc) return rc;
     return gbk_finish(ctx);
 }
@@ -849,7 +849,7 @@ extern "C" int gbkb200_gmodel_mcdisk_evaluate_f32(gbkb200_ctx* ctx, float cflux,
         }
     }
     if (ctx->mc_mode == 3 || ((ctx->mc_mode == 0 || ctx->mc_mode == 2) && !vec)) {
-        mcdisk_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, ctx->d_status);
+        mcdisk_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, gbk_status(ctx));
         GBK_CUDA_TRY(cudaGetLastError());
         return gbk_finish(ctx);
     }
@@ -860,7 +860,7 @@ extern "C" int gbkb200_gmodel_mcdisk_evaluate_f32(gbkb200_ctx* ctx, float cflux,
         float* lines = static_cast<float*>(ctx->mc_scratch);
         GBK_CUDA_TRY(cudaMemsetAsync(lines, 0, need, ctx->stream));
         mcdisk_v4_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, lines, nzp, copies,
-                                                          ctx->d_status);
+                                                          gbk_status(ctx));
         const dim3 tg((unsigned)((nsp + 63) / 64), (unsigned)((a.spec_size + 31) / 32));
         mc_lines_add_kernel<<<tg, 256, 0, ctx->stream>>>(lines, a.scube, nsp, nzp, a.spec_size,
                                                          copies);
@@ -897,7 +897,7 @@ extern "C" int gbkb200_gmodel_mcdisk_evaluate_f32(gbkb200_ctx* ctx, float cflux,
     f.ordata = ptrs[4]; f.ordata_cmp = ptrs[5];
     f.bound = bound;
     mcdisk_bound_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, bound);
-    mcdisk_fixed_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, f, ctx->d_status);
+    mcdisk_fixed_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, f, gbk_status(ctx));
     for (int i = 0; i < 6; ++i) {
         if (!lens[i]) continue;
         long long g = (lens[i] + 255) / 256;

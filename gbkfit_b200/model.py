@@ -577,6 +577,36 @@ class DModelMMaps:
                 for i, key in enumerate(self.keys())}
 
 
+STAGE_BYTES = 1 << 20     # outputs copied together; larger ones go one by one
+
+
+def to_host(out, stream):
+    """{key: {name: device tensor or None}} -> numpy arrays.  Small outputs
+    (maps) are copied through one pinned buffer with one wait: nine blocking
+    copies of 16 KB took 90 us."""
+    uniq = {}
+    for v in out.values():
+        for t in v.values():
+            if t is not None:
+                uniq.setdefault((t.data_ptr(), tuple(t.shape)), t)
+    if sum(t.numel() * t.element_size() for t in uniq.values()) > STAGE_BYTES or \
+            any(t.dtype != torch.float32 for t in uniq.values()):
+        return {k: {kk: (None if t is None else t.cpu().numpy()) for kk, t in v.items()}
+                for k, v in out.items()}
+    host = torch.empty(sum(t.numel() for t in uniq.values()), dtype=torch.float32,
+                       pin_memory=True)
+    views, off = {}, 0
+    with torch.cuda.stream(stream):
+        for key, t in uniq.items():
+            h = host[off:off + t.numel()].view(t.shape)
+            h.copy_(t, non_blocking=True)
+            views[key] = h.numpy()
+            off += t.numel()
+    stream.synchronize()
+    return {k: {kk: (None if t is None else views[t.data_ptr(), tuple(t.shape)].copy())
+                for kk, t in v.items()} for k, v in out.items()}
+
+
 class Model:
     """model/model.py: a (driver, dmodel, gmodel) triple."""
 
@@ -600,8 +630,7 @@ class Model:
 
     def evaluate_h(self, params, out_extra=None):
         out = self.evaluate_d(params, out_extra)
-        return {k: {kk: (None if vv is None else vv.cpu().numpy()) for kk, vv in v.items()}
-                for k, v in out.items()}
+        return to_host(out, self._driver.stream)
 
 
 class Objective:
