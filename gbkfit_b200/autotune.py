@@ -8,13 +8,8 @@ Knobs (all change speed only, never results beyond fp32 rounding):
   should stay in L2);
 * ``band``: output rows per PSF block of the direct mode (smaller bands: more
   resident blocks, more halo rows);
-* ``psf_variant``: PSF kernel sized for 4 or 5 resident blocks per SM, with
-  its residual in a separate pass or in the y-FIR items (data loaded after or
-  before each item's FIR), or persistent over all (set, plane) items;
-* ``model_variant``: the direct mode's model kernel (0: one 32-column chunk
-  per warp; 1: two chunks per warp on packed FP32 pairs; 2: a 4 x 8 spaxel
-  tile per warp; 3: 2 with the range-table masks by bit transposes; the
-  same values; 4: 3 with the line exponent from one multiply-add, the same
+* ``model_variant``: the direct mode's model kernel (3: a 4 x 8 spaxel tile
+  per warp; 4: the same with the line exponent from one multiply-add, the same
   values up to fp32 rounding);
 * ``rows_k1``: spectral rows per shared-memory group of the model kernel.
 
@@ -124,16 +119,9 @@ def tune_batched(w, data, err, nsets, budget_s=60.0, use_cache=True):
             t = time_config(w, data, err, nsets, cfg)
             if t < best_dt:
                 best_d, best_dt = cfg, t
-        # the PSF kernel's variants (resident blocks per SM x epilogue)
-        base = dict(best_d)
-        for variant in range(1, 8):
-            cfg = dict(base, psf_variant=variant)
-            t = time_config(w, data, err, nsets, cfg)
-            if t < best_dt:
-                best_d, best_dt = cfg, t
         # the model kernel's variants
         base = dict(best_d)
-        for mv in (1, 2, 3, 4):
+        for mv in (3, 4):
             cfg = dict(base, model_variant=mv)
             t = time_config(w, data, err, nsets, cfg)
             if t < best_dt:

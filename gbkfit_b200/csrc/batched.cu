@@ -503,6 +503,16 @@ static int trimmed_taps(const double* a, int n)
     return t;
 }
 
+// Sets per wave where the caller leaves it open: as many as 256 MB of scratch
+// hold, at least 8.  Waves of 8 sets leave the chip idle at their ends and
+// pay two launches each (32 sets of 48 x 44 x 32: four waves 60 us, one 28);
+// larger cubes fill it with 8, and beyond 256 MB only memory grows.
+static int auto_chunk(const gbkb200_batch* bt, size_t bytes_per_set)
+{
+    const size_t n = std::max<size_t>(8, (256u << 20) / std::max<size_t>(bytes_per_set, 1));
+    return (int)std::min<size_t>(n, bt->max_sets);
+}
+
 // Direct-mode setup: reversed FIR coefficients, plane buffers, the data's
 // summed-area table and shared memory sizes.  Returns
 // GBKB200_ERR_UNSUPPORTED when the direct path does not apply (PSF rank or
@@ -558,6 +568,9 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     for (int s = 0; s < P.Kx; ++s) vr[s] = (float)d->psf_v[d->kernel_size[0] - 1 - tx - s];
     for (int t = 0; t < P.Ky; ++t) ur[t] = (float)d->psf_u[d->kernel_size[1] - 1 - ty - t];
     for (int t = 0; t < P.Kz; ++t) lr[t] = (float)d->lsf[d->kernel_size[2] - 1 - tz - t];
+    if (d->chunk <= 0)
+        bt->chunk = auto_chunk(bt, (size_t)P.Nz * P.Wy * (P.pitch * sizeof(float) +
+                                                          P.nch * sizeof(int)));
     const size_t nrows = (size_t)bt->chunk * P.Nz * P.Wy;
     for (int i = 0; i < 33; ++i) {
         P.vr[i] = i < P.K ? vr[i] : 0.f;
@@ -633,6 +646,7 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     // sub-wave: 1381 / 1107 / 1008 / 972 us; the passes are bound by issue and
     // small launches leave the chip idle); beyond that only memory grows
     const size_t per_set = (size_t)P.Nz * K.ngw * KP_L * K.hxp * sizeof(float2);
+    if (d->chunk <= 0) bt->chunk = auto_chunk(bt, per_set);
     bt->wave = (int)std::max<size_t>(1, std::min<size_t>(bt->chunk, (256u << 20) / per_set));
     // tables, in 64-bit arithmetic: twiddles of both axes and the
     // spectrum of the PSF image shifted by its last tap to the origin, so that

@@ -362,7 +362,7 @@ typedef struct {
     const float* obs_m;     /* device: mask, or NULL */
     float weight;
     int max_sets;           /* largest nsets of an evaluate call */
-    int chunk;              /* sets per pipeline wave (0 = 8) */
+    int chunk;              /* sets per pipeline wave (0 = automatic: 256 MB of scratch, >= 8) */
     int rows_k1;            /* spectral rows per shared-memory group of the model kernel (0 = 16) */
     int rows_k5;            /* rows per block of the residual kernel (0 = 8) */
     int conv_mode;          /* 0 = automatic, 1 = FFT, 2 = direct separable FIR */
@@ -370,23 +370,12 @@ typedef struct {
     const double* psf_u;    /* host: (psf_rank, kernel_size[1]) */
     const double* psf_v;    /* host: (psf_rank, kernel_size[0]) */
     int psf_band;           /* direct mode: output rows per PSF block (0 = automatic) */
-    int psf_variant;        /* direct mode: PSF kernel variant 0-7: resident blocks per SM
-                             * (0-2: 4, 3-5: 5) x epilogue (variant % 3: 0 residual pass,
-                             * 1 residual in the y-FIR items, 2 as 1 with the data
-                             * prefetched); 6 = 0 as a persistent kernel (one resident
-                             * wave of blocks over all items, each item's range entries
-                             * copied in while the previous item runs); 7 = 0 on
-                             * 256-thread blocks with twice the shared memory (2 blocks
-                             * per SM); 0 = the first */
-    int model_variant;      /* direct mode, the model kernel (0-3 give the same values):
-                             * 0 = a warp per 32-column chunk stepping every lane through
-                             * the union of the lanes' channel windows; 1 = two chunks per
-                             * warp on packed FP32 pairs; 2 = a warp per 4 x 8 spaxel tile
-                             * (shorter channel unions); 3 = 2 with the range-table masks
-                             * from one bit transpose per 32 planes instead of a ballot
-                             * per plane; 4 = 3 with the line's exponent as -t^2, t one
-                             * multiply-add per channel (the same values up to fp32
-                             * rounding) */
+    int psf_variant;        /* 0-7: accepted; one PSF kernel is left */
+    int model_variant;      /* the model kernel: 0-3 the tile kernel (a warp per 4 x 8
+                             * spaxel tile; a warp per 32-column chunk above 2048
+                             * planes, which 2-4 refuse in the direct mode), 4 the same
+                             * with the line's exponent as -t^2, t one multiply-add per
+                             * channel (equal up to fp32 rounding) */
 } gbkb200_batch_desc;
 
 int gbkb200_batch_create(gbkb200_ctx* ctx, const gbkb200_batch_desc* desc, gbkb200_batch** out);
