@@ -544,15 +544,27 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     const int NW = (P.K + KB_XS - 1 + 3) / 4;
     P.pitch = (P.Wx + 31) / 32 * 32;
     P.nch = (P.Wx + 31) / 32;
+    if (d->chunk <= 0)
+        bt->chunk = auto_chunk(bt, (size_t)P.Nz * P.Wy * (P.pitch * sizeof(float) +
+                                                          P.nch * sizeof(int)));
     P.nwfast = nodewise(d) ? 1 : 0;
-    int band = d->psf_band > 0 ? std::min(d->psf_band, P.Ny) : P.Ny;
-    P.nbands = (P.Ny + band - 1) / band;
-    P.band = (P.Ny + P.nbands - 1) / P.nbands;
     // shared memory of a PSF block: rows of one pass at the widest box pitch;
     // at least K + 15 rows (8 output rows a pass), at most the whole band,
-    // otherwise 54 KB (four blocks per SM)
+    // otherwise 55 KB (four blocks per SM), where the boxes of a plane mostly fit.
+    // Planes over 180 KB take several passes, each with its K - 1 halo rows:
+    // 74 KB then (64 sets of 256 x 240 x 128: 987 -> 851 us; 512 sets of 128 x
+    // 128 x 96, 99 KB a plane, 1081 -> 1141 us), and up to three bands where the
+    // launch has few blocks (16 such sets: 324 -> 291 us).
     int bpmax = 4 * (KB_XS / 4 * (((P.Nx + 3) / 4 + KB_XS / 4 - 1) / (KB_XS / 4) - 1) + NW);
     bpmax += ((4 - bpmax % 32) + 32) % 32;
+    const bool wide = (long long)(P.Ny + P.K + 7) * bpmax * 4 > 180 * 1024;
+    int bands = 1;
+    if (d->psf_band > 0)
+        bands = (P.Ny + std::min(d->psf_band, P.Ny) - 1) / std::min(d->psf_band, P.Ny);
+    else if (wide)
+        bands = (int)std::min<long long>(3, 1 + 4440 / ((long long)std::max(1, bt->chunk) * P.Nz));
+    P.band = (P.Ny + bands - 1) / bands;
+    P.nbands = (P.Ny + P.band - 1) / P.band;
     // range entries of the band's input rows
     const long long xr_bytes = (long long)(P.band + P.K - 1) * P.nch * sizeof(int);
     const long long need_min = (long long)(P.K + 15) * bpmax;
@@ -560,7 +572,7 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     // psf_variant chose among forms of the PSF kernel that were slower at every
     // size; its values are accepted and mean the same kernel
     if (d->psf_variant < 0 || d->psf_variant > 7) return GBKB200_ERR_INVALID_ARG;
-    const long long cap = std::max(need_min, std::min(need_all, (55LL * 1024 - xr_bytes) / 4));
+    const long long cap = std::max(need_min, std::min(need_all, ((wide ? 74LL : 55LL) * 1024 - xr_bytes) / 4));
     if (cap * (long long)sizeof(float) + xr_bytes > 227LL * 1024) return GBKB200_ERR_UNSUPPORTED;
     P.cap = (int)cap;
     bt->smemB = (size_t)cap * sizeof(float) + (size_t)xr_bytes;
@@ -568,9 +580,6 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     for (int s = 0; s < P.Kx; ++s) vr[s] = (float)d->psf_v[d->kernel_size[0] - 1 - tx - s];
     for (int t = 0; t < P.Ky; ++t) ur[t] = (float)d->psf_u[d->kernel_size[1] - 1 - ty - t];
     for (int t = 0; t < P.Kz; ++t) lr[t] = (float)d->lsf[d->kernel_size[2] - 1 - tz - t];
-    if (d->chunk <= 0)
-        bt->chunk = auto_chunk(bt, (size_t)P.Nz * P.Wy * (P.pitch * sizeof(float) +
-                                                          P.nch * sizeof(int)));
     const size_t nrows = (size_t)bt->chunk * P.Nz * P.Wy;
     for (int i = 0; i < 33; ++i) {
         P.vr[i] = i < P.K ? vr[i] : 0.f;
