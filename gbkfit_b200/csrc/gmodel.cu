@@ -713,23 +713,41 @@ __global__ void __launch_bounds__(256) mcdisk_fixed_kernel(DiskArgs a, McArgs m,
     const double km = ldexp(1.0, fixed_shift(f.bound[1], m.nclouds));
     const CloudRange cr = block_clouds(m);
     int row = first_row(m, cr.begin + (int)threadIdx.x);
-    for (int ci = cr.begin + (int)threadIdx.x; ci < cr.end; ci += (int)blockDim.x) {
-        int x, y, z;
+    const int lane = threadIdx.x & 31;
+    for (int base = cr.begin; base < cr.end; base += (int)blockDim.x) {
+        const int ci = base + (int)threadIdx.x;
+        int x = 0, y = 0, z = 0;
         SpaxelOut o;
-        if (!mcdisk_cloud(a, m, mk, ci, row, x, y, z, o, bad)) continue;
-        const long long sp = x + (long long)a.sx * y;
-        if (f.image) fixed_add(&f.image[sp], o.orv, km);
-        int zlo, zhi;
-        if (f.scube && mc_line_window(o.vv, o.dv, a.spec_size, mk.ispec, a.spec_zero, zlo, zhi)) {
-            float amp, rinv;
-            mc_line_consts(o.dv, amp, rinv);
-            const long long plane = (long long)a.sx * a.sy;
-            for (int zs = zlo; zs <= zhi; ++zs) {
-                const float zv = a.spec_zero + zs * a.spec_step;
-                const float d = zv - o.vv;
-                fixed_add(&f.scube[sp + plane * zs], o.orv * (amp * line_e2(d, rinv)), kc);
+        const bool on = ci < cr.end && mcdisk_cloud(a, m, mk, ci, row, x, y, z, o, bad);
+        const int sp = x + a.sx * y;
+        if (f.scube) {
+            // the warp's clouds one after the other, a lane per channel: the
+            // additions of a line meet in a few L2 sectors
+            int zlo = 0, zhi = -1;
+            float amp = 0.f, rinv = 0.f;
+            if (on && mc_line_window(o.vv, o.dv, a.spec_size, mk.ispec, a.spec_zero, zlo, zhi))
+                mc_line_consts(o.dv, amp, rinv);
+            else
+                zhi = -1;
+            for (unsigned todo = __ballot_sync(0xffffffffu, zlo <= zhi); todo; todo &= todo - 1) {
+                const int k = __ffs(todo) - 1;
+                const int lo = __shfl_sync(0xffffffffu, zlo, k);
+                const int hi = __shfl_sync(0xffffffffu, zhi, k);
+                const float vk = __shfl_sync(0xffffffffu, o.vv, k);
+                const float ok = __shfl_sync(0xffffffffu, o.orv, k);
+                const float ak = __shfl_sync(0xffffffffu, amp, k);
+                const float rk = __shfl_sync(0xffffffffu, rinv, k);
+                long long* col = f.scube +
+                                 (long long)__shfl_sync(0xffffffffu, sp, k) * a.spec_size;
+                for (int zs = lo + lane; zs <= hi; zs += 32) {
+                    const float zv = a.spec_zero + zs * a.spec_step;
+                    const float d = zv - vk;
+                    fixed_add(&col[zs], ok * (ak * line_e2(d, rk)), kc);
+                }
             }
         }
+        if (!on) continue;
+        if (f.image) fixed_add(&f.image[sp], o.orv, km);
         const long long idx = idx3(x, y, z, a.sx, a.sy);
         // last-writer-wins assignments, racy as in the reference
         if (a.wdata) a.wdata[idx] = o.wv;
@@ -742,6 +760,33 @@ __global__ void __launch_bounds__(256) mcdisk_fixed_kernel(DiskArgs a, McArgs m,
         if (a.ddata_cmp) a.ddata_cmp[idx] = o.dv;
     }
     if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
+}
+
+// scube[z][s] += acc[s][z] / 2^k (32 x 32 tiles)
+__global__ void __launch_bounds__(256) fixed_lines_to_float_kernel(const long long* acc,
+                                                                   float* out, long long nsp,
+                                                                   int nz, const unsigned* bound,
+                                                                   int nclouds)
+{
+    __shared__ float tile[32][33];
+    const double inv = ldexp(1.0, -fixed_shift(bound[0], nclouds));
+    const long long s0 = (long long)blockIdx.x * 32;
+    const int z0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) {
+        const long long s = s0 + ty + k;
+        const int z = z0 + tx;
+        const long long v = s < nsp && z < nz ? acc[s * nz + z] : 0;
+        tile[ty + k][tx] = (float)((double)v * inv);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) {
+        const long long s = s0 + tx;
+        const int z = z0 + ty + k;
+        const float v = tile[tx][ty + k];
+        if (s < nsp && z < nz && v != 0.f) out[(long long)z * nsp + s] += v;
+    }
 }
 
 // out[i] += acc[i] / 2^k
@@ -946,12 +991,17 @@ extern "C" int gbkb200_gmodel_mcdisk_evaluate_f32(gbkb200_ctx* ctx, float cflux,
     f.bound = bound;
     mcdisk_bound_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, bound);
     mcdisk_fixed_kernel<<<blocks, 256, 0, ctx->stream>>>(a, m, f, gbk_status(ctx));
-    for (int i = 0; i < 6; ++i) {
+    if (ncube) {
+        const dim3 tg((unsigned)((nsp + 31) / 32), (unsigned)((a.spec_size + 31) / 32));
+        fixed_lines_to_float_kernel<<<tg, 256, 0, ctx->stream>>>(f.scube, a.scube, nsp,
+                                                                 a.spec_size, bound, nclouds);
+    }
+    for (int i = 1; i < 6; ++i) {
         if (!lens[i]) continue;
         long long g = (lens[i] + 255) / 256;
         if (g > 148 * 8) g = 148 * 8;
-        fixed_to_float_kernel<<<(int)g, 256, 0, ctx->stream>>>(ptrs[i], outs[i], lens[i], bound,
-                                                             i == 0 ? 0 : 1, nclouds);
+        fixed_to_float_kernel<<<(int)g, 256, 0, ctx->stream>>>(ptrs[i], outs[i], lens[i], bound, 1,
+                                                             nclouds);
     }
     GBK_CUDA_TRY(cudaGetLastError());
     return gbk_finish(ctx);
