@@ -309,11 +309,9 @@ static int get_plan(FftState* st, const Size3& s, Plan** out)
     if ((rc = make_axis(p.ax, M))) return rc;
     if ((rc = make_axis(p.ay, p.ny))) return rc;
     if ((rc = make_axis(p.az, p.nz))) return rc;
-    if (st->mode == 0) {
-        if (p.nx % 2 == 0) p.fx = fast_rows(M);
-        p.fy = fast_lines(p.ny);
-        p.fz = fast_lines(p.nz);
-    }
+    if (p.nx % 2 == 0) p.fx = st->mode == 0 ? fast_rows(M) : mixed_rows(M);
+    p.fy = st->mode == 0 ? fast_lines(p.ny) : mixed_lines(p.ny);
+    p.fz = st->mode == 0 ? fast_lines(p.nz) : mixed_lines(p.nz);
     std::vector<float2> post(p.hx);
     for (int k = 0; k < p.hx; ++k) {
         double ang = -2.0 * M_PI * (double)k / (double)p.nx;

@@ -1,5 +1,6 @@
-"""The two-factor line transforms of the FFT convolution against numpy's
-64-bit transforms, at every instantiated length and on grids whose rows do
+"""The two-factor line transforms of the FFT convolution (mode 0) and the
+mixed-radix passes at compile-time lengths (mode 1) against numpy's 64-bit
+transforms, at every instantiated length and on grids whose rows do
 not fill a block's 16 columns or 16 rows."""
 
 import numpy as np
@@ -28,12 +29,14 @@ def _rel(a, b):
     (224, 224, 2), (256, 256, 2), (288, 288, 3), (320, 320, 2), (352, 352, 1), (384, 384, 1),
     (32, 3, 160), (64, 5, 192), (32, 1, 224), (32, 3, 256), (96, 1, 288), (32, 2, 320),
     (32, 1, 352), (34, 2, 384), (24, 32, 20), (31, 64, 32), (416, 32, 32)])
-def test_transforms_and_convolution(size):
+@pytest.mark.parametrize('mode', [0, 1])
+def test_transforms_and_convolution(size, mode):
     nx, ny, nz = size
     rng = np.random.default_rng(nx + 1000 * ny + 1000000 * nz)
     a = rng.standard_normal((nz, ny, nx)).astype(np.float32)
     k = rng.standard_normal((nz, ny, nx)).astype(np.float32)
     fft = DriverB200(0).backends().fft(np.float32)
+    fft._ctx.set_fft(mode)
     spec = np.fft.rfftn(a.astype(np.float64))
     ar = torch.from_numpy(a).cuda()
     ac = torch.zeros((nz, ny, nx // 2 + 1), dtype=torch.complex64, device='cuda')
