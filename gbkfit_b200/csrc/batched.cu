@@ -544,6 +544,7 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     const int NW = (P.K + KB_XS - 1 + 3) / 4;
     P.pitch = (P.Wx + 31) / 32 * 32;
     P.nch = (P.Wx + 31) / 32;
+    P.nch_inv = P.nch > 1 ? (unsigned)(((1ull << 32) + P.nch - 1) / P.nch) : 0u;
     if (d->chunk <= 0)
         bt->chunk = auto_chunk(bt, (size_t)P.Nz * P.Wy * (P.pitch * sizeof(float) +
                                                           P.nch * sizeof(int)));

@@ -43,6 +43,8 @@ struct BatchKernelArgs {
     float lsfr[33];       // (Kz): LSF reversed
     float* mplanes;       // (chunk, Nz, Wy, pitch): written where xr is not empty
     int nch;              // 32-column chunks per window row, ceil(Wx / 32)
+    unsigned nch_inv;     // ceil(2^32 / nch), nch > 1: i / nch = umulhi(i, nch_inv) for
+                          // i nch < 2^32
     int nwfast;           // the disk's traits are exactly rpt/vpt/dpt uid 101 (smdisk_spaxel_nw)
     int* xrt;             // (chunk, Nz, Wy, nch): the nonzero columns of each plane row
                           // chunk as a 32-bit mask (bit j: column 32 chunk + j; 0: the
@@ -461,27 +463,28 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
         s_box[0] = INT_MAX; s_box[1] = -1; s_box[2] = INT_MAX; s_box[3] = -1;
     }
     __syncthreads();
-    // bounding box of the nonzero input row chunks: a thread per row
+    // bounding box of the nonzero input row chunks, all of a thread's entries
+    // requested at once
     {
         int y0 = INT_MAX, y1 = -1, x0 = INT_MAX, x1 = -1;
-        for (int r = threadIdx.x; r < in1 - ob0; r += NT) {
-            const int* src = xr + (ob0 + r) * P.nch;
-            int* dst = s_xr + r * P.nch;
-            int first = INT_MAX, last = -1;
-#pragma unroll 4
-            for (int ch = 0; ch < P.nch; ++ch) {
-                const int v = src[ch];
-                dst[ch] = v;
-                if (v != 0) {
-                    first = min(first, ch * 32 + __ffs(v) - 1);
-                    last = ch * 32 + 31 - __clz(v);
+        const int* src = xr + ob0 * P.nch;
+        const int n = (in1 - ob0) * P.nch;
+        for (int i0 = threadIdx.x; i0 < n; i0 += 8 * NT) {
+            int v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = i0 + u * NT < n ? src[i0 + u * NT] : 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int i = i0 + u * NT;
+                if (i < n) s_xr[i] = v[u];
+                if (v[u] != 0) {
+                    const int r = P.nch == 1 ? i : (int)__umulhi((unsigned)i, P.nch_inv);
+                    const int ch = i - r * P.nch;
+                    y0 = min(y0, ob0 + r);
+                    y1 = max(y1, ob0 + r);
+                    x0 = min(x0, ch * 32 + __ffs(v[u]) - 1);
+                    x1 = max(x1, ch * 32 + 31 - __clz(v[u]));
                 }
-            }
-            if (last >= 0) {
-                y0 = min(y0, ob0 + r);
-                y1 = ob0 + r;
-                x0 = min(x0, first);
-                x1 = max(x1, last);
             }
         }
         y0 = __reduce_min_sync(0xffffffffu, y0);
@@ -568,8 +571,9 @@ __global__ void __launch_bounds__(KB_THREADS, 4) kb_psf_residual(BatchKernelArgs
                 for (int i = (ly1 + 1 - ys) * bp4 + threadIdx.x; i < (rend - ys) * bp4; i += NT)
                     sm4[i] = z;
         }
+        // a warp's x FIR reads only the rows that the warp has loaded
         cp_async_wait_all();
-        __syncthreads();
+        __syncwarp();
         // x FIR in place: S[y][xo] = sum_s vr[s] S[y][xo + s].  A warp owns whole
         // rows (ly0 + warp, + NWARPS, ...); its lanes take consecutive (row,
         // strip) pairs of those rows, 32 per pass.  Strip g writes columns
