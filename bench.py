@@ -912,6 +912,18 @@ def run_serving(args):
                 higher_is_better=True, dtype='f32', data='synthetic', serving=out)
 
 
+def reference_available():
+    """Whether the compiled reference templates are there or can be built
+    (they need the reference's sources)."""
+    from oracle.oracle import Reference, build
+    if not Reference.available():
+        try:
+            build()
+        except (OSError, subprocess.CalledProcessError):
+            pass
+    return Reference.available()
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument('--gpus', type=int, default=1)
@@ -946,6 +958,13 @@ def main():
                     help='smdisk_batch128 is the headline; the others print their own line')
     ap.add_argument('--requests', type=int, default=10000, help='serving workload: requests')
     args = ap.parse_args()
+    if args.impl == 'reference' and not reference_available():
+        if int(os.environ.get('RANK', 0)) == 0:
+            print(json.dumps(dict(impl='reference', unavailable='the reference sources are not '
+                                  'there to build its templates from')))
+        return
+    if args.cpu_baseline and args.impl != 'reference' and not reference_available():
+        args.cpu_baseline = False       # cpu_baseline: null
     if args.warmup < 3:
         args.warmup = 3
     other = dict(mcdisk_cube256=run_mcdisk, smdisk_cube64=run_smdisk64, grad96=run_grad96,
