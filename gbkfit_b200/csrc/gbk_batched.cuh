@@ -265,8 +265,12 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf(B
 // s = sqrt(log2(e) / (2 sigma^2)), one multiply-add and one multiply per
 // channel instead of a multiply-add, an add and two multiplies; the same line
 // up to fp32 rounding (not bit-identical to the other forms).
+// Ten blocks a SM (48 registers, 36 bytes spilled before the channel loop): 512
+// sets of 128 x 128 x 96 in 472 us, 490 with eight and 64 registers, 473 with
+// nine, 480 with twelve; at 15 taps 67.5, 68.2, 71.4 and 70.6 us (16 sets of 256 x
+// 240 x 128).
 template<int KZ, bool SL>
-__global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf_t(BatchKernelArgs P, int* status)
+__global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 10 : 4)) ka_lines_lsf_t(BatchKernelArgs P, int* status)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rg = blockIdx.x / P.nch, chunk = blockIdx.x % P.nch;   // grid: ceil(Wy / 4) nch
