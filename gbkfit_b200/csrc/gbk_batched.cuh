@@ -433,10 +433,18 @@ __device__ __forceinline__ void kb_zero_rows(float* m, int nx, bool vec, int r0,
 //     the rows that the y FIR reads is zeroed;
 //   - x FIR in place, a warp per row, its lanes on consecutive (row, strip)
 //     pairs of its rows, 12 outputs per lane window;
-//   - y FIR, 8 x 4 outputs per (8-row group, column) item in registers, and
-//     in the same item the crop, residual (objective.hpp:7-31) and r^2
-//     against the data.
+//   - y FIR, 8 x 4 outputs per (8-row group, column) item in registers, in
+//     place; then the crop, residual (objective.hpp:7-31) and r^2 against the
+//     data.
 // The zero-model residual outside the box comes from the summed-area table.
+//
+// Bound by issue (59 % of cycles) and shared-memory wavefronts (63 %) with 16
+// warps a SM; a block's phases (cycles, 512 sets of 128 x 128 x 96): box 3.0k, to
+// the loads 1.4k, loads 7.0k, x FIR 5.3k, y FIR 4.9k, residual 6.0k.  That batch:
+// 1282 us with run-time divisions in the loads and outside the box and
+// two-way bank conflicts in 8-column strips, 1037 now; 100 sets of 97 x 83 x 61
+// 191 -> 106.  160 to 256 threads a block 1216-1300 us, 3, 5 or 6 blocks a SM
+// 1141, 1090, 1199.
 constexpr int KB_THREADS = 128;
 constexpr int KB_XS = 12;       // output columns of an x FIR strip
 constexpr int KB_NX_MAX = 512;  // widest data cube of the direct mode
