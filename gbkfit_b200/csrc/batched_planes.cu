@@ -10,7 +10,7 @@ static bool rows_fit(int w, PlaneRows& f)
     constexpr int n = N1 * 16;
     if (n < w) return false;
     f.n = n;
-    f.threads = KP_P * (N1 > 16 ? N1 : 16);
+    f.threads = kp_threads(N1);
     f.smem = (size_t)(KP_P * N1 * 17 + n) * sizeof(float2);
     f.rows = kp_rows<N1>;
     f.resid = kp_resid<N1>;

@@ -55,6 +55,11 @@ __device__ __forceinline__ unsigned plane_groups(const PlaneArgs& P, long long p
 }
 
 constexpr int KP_P = KP_L / 2;        // row pairs per block
+// threads of the row kernels: whole warps (their sums shuffle across the warp)
+__host__ __device__ constexpr int kp_threads(int n1)
+{
+    return (KP_P * (n1 > 16 ? n1 : 16) + 31) / 32 * 32;
+}
 
 // Rows [16 g, 16 g + 16) of a plane, two real rows as the real and imaginary
 // part of one n = 16 N1 point transform:
@@ -63,9 +68,9 @@ constexpr int KP_P = KP_L / 2;        // row pairs per block
 // column of those is written); a thread's columns lie 16 apart, so that the
 // mask word of an element and its bit are known at compile time up to the lane.
 template<int N1>
-__global__ void __launch_bounds__(KP_P * (N1 > 16 ? N1 : 16)) kp_rows(PlaneArgs P)
+__global__ void __launch_bounds__(kp_threads(N1)) kp_rows(PlaneArgs P)
 {
-    constexpr int N2 = 16, n = N1 * N2, T = KP_P * (N1 > N2 ? N1 : N2), P2 = N2 + 1;
+    constexpr int N2 = 16, n = N1 * N2, T = kp_threads(N1), P2 = N2 + 1;
     extern __shared__ float2 sm[];          // 8 pairs of N1 P2, then n twiddles
     float2* s_tw = sm + KP_P * N1 * P2;
     __shared__ int s_mask[KP_L * (KP_MAX_W / 32)];
@@ -198,12 +203,12 @@ __global__ void __launch_bounds__(KP_L * (N1 > 16 ? N1 : 16)) kp_cols(PlaneArgs 
 // conj X1 + i conj X2 beyond n / 2), the first Nx columns, r = (m - d) iw
 // (objective.hpp:7-31) and the block's sum of r^2.
 template<int N1>
-__global__ void __launch_bounds__(KP_P * (N1 > 16 ? N1 : 16)) kp_resid(PlaneArgs P)
+__global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
 {
-    constexpr int N2 = 16, n = N1 * N2, T = KP_P * (N1 > N2 ? N1 : N2), P2 = N2 + 1;
+    constexpr int N2 = 16, n = N1 * N2, T = kp_threads(N1), P2 = N2 + 1;
     extern __shared__ float2 sm[];          // 8 pairs of N1 P2, then n twiddles
     float2* s_tw = sm + KP_P * N1 * P2;
-    __shared__ float s_part[(T + 31) / 32];
+    __shared__ float s_part[T / 32];
     const int zo = blockIdx.y, y0 = blockIdx.x * KP_L, rows = min(KP_L, P.Ny - y0);
     const long long plane = (long long)blockIdx.z * P.Nz + zo;
     const int b = P.set0 + blockIdx.z;
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(KP_P * (N1 > 16 ? N1 : 16)) kp_resid(PlaneArgs
     __syncthreads();
     if (threadIdx.x == 0) {
         float s = 0.f;
-        for (int w = 0; w < (T + 31) / 32; ++w) s += s_part[w];
+        for (int w = 0; w < T / 32; ++w) s += s_part[w];
         P.partials[((long long)b * P.Nz + zo) * gridDim.x + blockIdx.x] = (double)s;
     }
 }

@@ -28,6 +28,9 @@ def _workload(size, nsets, fwhm, lsf_fwhm, seed):
 @pytest.mark.parametrize('size,fwhm,lsf,planes', [
     ((48, 48, 20), 1.15, 1.5, 1), ((49, 47, 20), 1.15, 1.5, 1), ((80, 16, 12), 1.15, 1.5, 1),
     ((33, 64, 200), 1.15, 1.0, 1), ((54, 35, 16), 3.0, 2.0, 1), ((150, 150, 9), 3.0, 1.5, 1),
+    # every transform length of 16 N1 points with N1 > 12 along x and along y
+    *[((16 * n1 - 16, 18, 5), 1.15, 1.5, 1) for n1 in (14, 15, 16, 18, 20, 22, 24)],
+    *[((18, 16 * n1 - 16, 5), 1.15, 1.5, 1) for n1 in (14, 15, 16, 18, 20, 22, 24)],
     ((342, 20, 8), 3.0, 1.5, 1), ((20, 341, 8), 3.0, 1.5, 1),
     ((40, 36, 24), 1.5, 6.0, 0), ((343, 24, 6), 3.0, 1.5, 0)])
 def test_planewise_vs_oracle(gpu, oracle_built, size, fwhm, lsf, planes):
