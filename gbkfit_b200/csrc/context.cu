@@ -1,6 +1,7 @@
 // Context (module object) management and error reporting of the C ABI.
 #include "gbk_common.cuh"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -161,21 +162,31 @@ extern "C" const char* gbkb200_last_cuda_error(void)
 }
 
 namespace {
+struct SmemLimit {
+    size_t dyn = 0;             // dynamic bytes a launch may ask for now
+    bool known = false;
+};
 std::mutex g_smem_mutex;
-std::map<std::pair<int, const void*>, size_t> g_smem_limits;   // (device, kernel) -> bytes
+std::map<std::pair<int, const void*>, SmemLimit> g_smem_limits;   // by (device, kernel)
 }  // namespace
 
 int gbk_raise_smem_limit(const void* fn, size_t bytes)
 {
-    if (bytes <= 48 * 1024) return GBKB200_OK;      // the default limit
     int dev = 0;
     GBK_CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(g_smem_mutex);
-    size_t& cur = g_smem_limits[{dev, fn}];
-    if (bytes > cur) {
+    SmemLimit& lim = g_smem_limits[{dev, fn}];
+    if (!lim.known) {
+        // the default of 48 KB holds for the kernel's static and dynamic bytes together
+        cudaFuncAttributes a;
+        GBK_CUDA_TRY(cudaFuncGetAttributes(&a, fn));
+        lim.dyn = 48 * 1024 - std::min<size_t>(a.sharedSizeBytes, 48 * 1024);
+        lim.known = true;
+    }
+    if (bytes > lim.dyn) {
         GBK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)bytes));
-        cur = bytes;
+        lim.dyn = bytes;
     }
     return GBKB200_OK;
 }
