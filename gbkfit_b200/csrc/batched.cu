@@ -506,11 +506,12 @@ static int trimmed_taps(const double* a, int n)
 // Sets per wave where the caller leaves it open: as many as 256 MB of scratch
 // hold, at least 8.  Waves of 8 sets leave the chip idle at their ends and
 // pay two launches each (32 sets of 48 x 44 x 32: four waves 60 us, one 28);
-// larger cubes fill it with 8, and beyond 256 MB only memory grows.
+// larger cubes fill it with 8, and beyond 256 MB only memory grows.  No more than
+// 65535: the sets of a wave are a y or z grid dimension.
 static int auto_chunk(const gbkb200_batch* bt, size_t bytes_per_set)
 {
     const size_t n = std::max<size_t>(8, (256u << 20) / std::max<size_t>(bytes_per_set, 1));
-    return (int)std::min<size_t>(n, bt->max_sets);
+    return (int)std::min<size_t>(std::min<size_t>(n, 65535), bt->max_sets);
 }
 
 // Direct-mode setup: reversed FIR coefficients, plane buffers, the data's
