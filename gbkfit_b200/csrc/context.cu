@@ -37,7 +37,7 @@ int gbk_finish(gbkb200_ctx* ctx)
         return GBKB200_ERR_CUDA;
     }
     if (!ctx->sync) return GBKB200_OK;
-    // the first wait after asynchronous calls reads the device's word as well
+    // a context that was ever asynchronous: the device's word as well
     if (ctx->async_calls) return gbkb200_ctx_synchronize(ctx);
     GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return take_mapped_status(ctx);
@@ -130,7 +130,6 @@ extern "C" int gbkb200_ctx_synchronize(gbkb200_ctx* ctx)
     GBK_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
     GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (ctx->sync) ctx->async_calls = 0;
     int s = *ctx->h_status;
     if (s) {
         GBK_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));

@@ -70,7 +70,8 @@ struct gbkb200_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     int sync = 1;
-    int async_calls = 0;          // calls may have been made in asynchronous mode
+    int async_calls = 0;          // was in asynchronous mode at some time: its calls, or graphs
+                                  // captured then and replayed later, write d_status
     unsigned long long seed = 42;
     int mc_mode = 0;
     int fft_mode = 0;             // 1: mixed-radix passes only (gbkb200_ctx_set_fft)
