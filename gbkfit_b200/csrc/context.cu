@@ -20,13 +20,13 @@ static int status_code(int s)
     return GBKB200_ERR_INVALID_ARG;
 }
 
-// reads and clears the mapped word (the stream has been waited for)
+// reads and clears the mapped word (the stream has been waited for): its bits
 static int take_mapped_status(gbkb200_ctx* ctx)
 {
     volatile int* w = ctx->h_status + 1;
     const int s = *w;
     if (s) *w = 0;
-    return status_code(s);
+    return s;
 }
 
 int gbk_finish(gbkb200_ctx* ctx)
@@ -40,7 +40,7 @@ int gbk_finish(gbkb200_ctx* ctx)
     // a context that was ever asynchronous: the device's word as well
     if (ctx->async_calls) return gbkb200_ctx_synchronize(ctx);
     GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return take_mapped_status(ctx);
+    return status_code(take_mapped_status(ctx));
 }
 
 extern "C" int gbkb200_ctx_create(gbkb200_ctx** out, int device)
@@ -130,14 +130,14 @@ extern "C" int gbkb200_ctx_synchronize(gbkb200_ctx* ctx)
     GBK_CUDA_TRY(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
     GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    int s = *ctx->h_status;
+    const int s = *ctx->h_status;
     if (s) {
         GBK_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
         GBK_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         *ctx->h_status = 0;
-        return status_code(s);
     }
-    return take_mapped_status(ctx);
+    // both words are cleared by the call that reports them
+    return status_code(s | take_mapped_status(ctx));
 }
 
 extern "C" const char* gbkb200_error_string(int code)

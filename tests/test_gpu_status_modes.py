@@ -63,3 +63,14 @@ def test_status_of_a_replayed_graph(gpu):
     with pytest.raises(_native.NativeError):
         c.good()
     c.good()
+
+
+def test_status_of_both_modes_at_once(gpu):
+    from gbkfit_b200 import _native
+    c = _Calls()
+    c.ctx.set_sync(False)
+    c.bad()
+    c.ctx.set_sync(True)
+    with pytest.raises(_native.NativeError):
+        c.bad()
+    c.good()
