@@ -18,6 +18,7 @@
 //    two-pass fixed-point accumulation (mode 1, deterministic).
 #include "gbk_disk.cuh"
 
+#include <algorithm>
 #include <climits>
 
 namespace gbk {
@@ -31,30 +32,31 @@ constexpr int THIN_Y = 2, THIN_Z = 8;
 __global__ void __launch_bounds__(32 * THIN_Y) smdisk_thin_kernel(DiskArgs a, int* status)
 {
     const int x = blockIdx.x * 32 + threadIdx.x;
-    const int y = blockIdx.y * THIN_Y + threadIdx.y;
-    const bool inside = x < a.sx && y < a.sy;
     int bad = 0;
     DiskConst kc = disk_const(a);
-    SpaxelOut o;
-    bool on = inside && smdisk_spaxel(a, kc, x, y, 0, o, bad);
-    int zlo = INT_MAX, zhi = -1;
-    float amp = 0, inv2c2 = 0;
-    if (on) {
-        if (a.image) a.image[x + (long long)a.sx * y] += o.orv;
-        smdisk_side_outputs(a, x, y, 0, o);
-        if (a.scube && line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
-            amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
-            inv2c2 = 2 * o.dv * o.dv;
-        } else {
-            zlo = INT_MAX;
-            zhi = -1;
+    // one pass, but for more rows than a grid dimension holds pairs (whole warps)
+    for (int y = blockIdx.y * THIN_Y + threadIdx.y; y < a.sy; y += gridDim.y * THIN_Y) {
+        SpaxelOut o;
+        bool on = x < a.sx && smdisk_spaxel(a, kc, x, y, 0, o, bad);
+        int zlo = INT_MAX, zhi = -1;
+        float amp = 0, inv2c2 = 0;
+        if (on) {
+            if (a.image) a.image[x + (long long)a.sx * y] += o.orv;
+            smdisk_side_outputs(a, x, y, 0, o);
+            if (a.scube &&
+                line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
+                amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
+                inv2c2 = 2 * o.dv * o.dv;
+            } else {
+                zlo = INT_MAX;
+                zhi = -1;
+            }
         }
-    }
-    // channel loop over the union of the warp's windows: coalesced rows
-    const unsigned full = 0xffffffffu;
-    int wlo = __reduce_min_sync(full, zlo);
-    int whi = __reduce_max_sync(full, zhi);
-    if (a.scube) {
+        // channel loop over the union of the warp's windows: coalesced rows
+        const unsigned full = 0xffffffffu;
+        int wlo = __reduce_min_sync(full, zlo);
+        int whi = __reduce_max_sync(full, zhi);
+        if (!a.scube) continue;
         const long long plane = (long long)a.sx * a.sy;
         float* col = a.scube + (x + (long long)a.sx * y);
         for (int z0 = wlo; z0 <= whi; z0 += THIN_Z) {
@@ -865,7 +867,8 @@ int gbk_launch_smdisk(const DiskArgs& a, cudaStream_t stream, int* status)
 {
     const bool thin = a.rht.uids == nullptr;
     if (thin && a.sz == 1) {
-        dim3 block(32, THIN_Y), grid((a.sx + 31) / 32, (a.sy + THIN_Y - 1) / THIN_Y);
+        dim3 block(32, THIN_Y),
+            grid((a.sx + 31) / 32, std::min((a.sy + THIN_Y - 1) / THIN_Y, 65535));
         smdisk_thin_kernel<<<grid, block, 0, stream>>>(a, status);
     } else {
         dim3 block(32, TH), grid((a.sx + 31) / 32, a.sy);
