@@ -565,17 +565,26 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
         bands = (P.Ny + std::min(d->psf_band, P.Ny) - 1) / std::min(d->psf_band, P.Ny);
     else if (wide)
         bands = (int)std::min<long long>(3, 1 + 4440 / ((long long)std::max(1, bt->chunk) * P.Nz));
-    P.band = (P.Ny + bands - 1) / bands;
-    P.nbands = (P.Ny + P.band - 1) / P.band;
-    // range entries of the band's input rows
-    const long long xr_bytes = (long long)(P.band + P.K - 1) * P.nch * sizeof(int);
-    const long long need_min = (long long)(P.K + 15) * bpmax;
-    const long long need_all = (long long)(P.band + P.K + 7) * bpmax;
     // psf_variant chose among forms of the PSF kernel that were slower at every
     // size; its values are accepted and mean the same kernel
     if (d->psf_variant < 0 || d->psf_variant > 7) return GBKB200_ERR_INVALID_ARG;
-    const long long cap = std::max(need_min, std::min(need_all, ((wide ? 74LL : 55LL) * 1024 - xr_bytes) / 4));
-    if (cap * (long long)sizeof(float) + xr_bytes > 227LL * 1024) return GBKB200_ERR_UNSUPPORTED;
+    bt->kb = kb_fn(P.K);
+    cudaFuncAttributes kb_attr;
+    GBK_CUDA_TRY(cudaFuncGetAttributes(&kb_attr, reinterpret_cast<const void*>(bt->kb)));
+    const long long room = 227LL * 1024 - (long long)kb_attr.sharedSizeBytes;
+    long long xr_bytes, cap;
+    for (;; ++bands) {
+        P.band = (P.Ny + bands - 1) / bands;
+        P.nbands = (P.Ny + P.band - 1) / P.band;
+        // range entries of the band's input rows
+        xr_bytes = (long long)(P.band + P.K - 1) * P.nch * sizeof(int);
+        const long long need_min = (long long)(P.K + 15) * bpmax;
+        const long long need_all = (long long)(P.band + P.K + 7) * bpmax;
+        cap = std::max(need_min, std::min(need_all, ((wide ? 74LL : 55LL) * 1024 - xr_bytes) / 4));
+        // more bands where a band of thousands of rows has too many entries
+        if (cap * (long long)sizeof(float) + xr_bytes <= room) break;
+        if (P.band <= 8) return GBKB200_ERR_UNSUPPORTED;
+    }
     P.cap = (int)cap;
     bt->smemB = (size_t)cap * sizeof(float) + (size_t)xr_bytes;
     std::vector<float> vr(P.K, 0.f), ur(P.K, 0.f), lr(P.Kz);
@@ -607,7 +616,6 @@ static int setup_direct(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     const bool fits = (long long)P.Nz * 16 <= 32 * 1024;
     if (d->model_variant >= 2 && !fits) return GBKB200_ERR_UNSUPPORTED;
     pick_ka(bt, d->model_variant, fits);
-    bt->kb = kb_fn(P.K);
     {
         const int rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->kb), bt->smemB);
         if (rc) return rc;
