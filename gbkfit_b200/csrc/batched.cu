@@ -720,7 +720,6 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
         cudaMalloc(&bt->pconv, (size_t)bt->wave * P.Nz * P.Ny * K.hxp * sizeof(float2)) !=
             cudaSuccess ||
         cudaMalloc(&bt->pflags, (size_t)bt->wave * P.Nz * 32) != cudaSuccess ||
-        cudaMalloc(&bt->iw, (size_t)P.Nz * P.Ny * P.Nx * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&bt->ptab, tab.size() * sizeof(float2)) != cudaSuccess ||
         cudaMalloc(&bt->partials, (size_t)bt->max_sets * bt->nper * sizeof(double)) != cudaSuccess)
         return GBKB200_ERR_OOM;
@@ -728,11 +727,7 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
                             cudaMemcpyHostToDevice));
     P.mplanes = bt->mplanes;
     P.xrt = bt->xrt;
-    P.iw = bt->iw;
     P.partials = bt->partials;
-    k_iw<<<592, 256, 0, bt->ctx->stream>>>(P, bt->iw, (long long)P.Nz * P.Ny * P.Nx);
-    GBK_CUDA_TRY(cudaGetLastError());
-    GBK_CUDA_TRY(cudaStreamSynchronize(bt->ctx->stream));
     K.mplanes = bt->mplanes;
     K.xrt = bt->xrt;
     K.work = bt->work;
@@ -742,7 +737,9 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     K.twy = K.twx + px;
     K.spec = K.twy + n;
     K.obs = P.obs;
-    K.iw = bt->iw;
+    K.err = P.err;
+    K.msk = P.msk;
+    K.weight = P.weight;
     K.partials = bt->partials;
     int rc;
     if ((rc = gbk_raise_smem_limit(reinterpret_cast<const void*>(bt->pr.rows), bt->pr.smem)) ||
@@ -1019,7 +1016,7 @@ extern "C" int gbkb200_batch_info(const gbkb200_batch* bt, int fft_size[3], int*
             const size_t nrows = (size_t)bt->wave * P.Nz * P.Wy;
             b += nrows * (P.pitch * sizeof(float) + P.nch * sizeof(int)) +
                  (size_t)bt->wave * P.Nz * (bt->K.ngw * KP_L + P.Ny) * bt->K.hxp * sizeof(float2) +
-                 (size_t)bt->wave * P.Nz * 32 + (size_t)P.Nz * P.Ny * P.Nx * sizeof(float) +
+                 (size_t)bt->wave * P.Nz * 32 +
                  ((size_t)bt->pr.n + (size_t)bt->pc.n * (1 + bt->K.hxp)) * sizeof(float2);
         } else {
             b += (size_t)bt->chunk * P.Wz * P.Py * P.hx * sizeof(float2) +
@@ -1078,7 +1075,8 @@ extern "C" int gbkb200_batch_evaluate(gbkb200_batch* bt, int nsets, const float*
     if (bt->planes) {
         PlaneArgs K = bt->K;
         K.model = model;
-        K.vec = vector_rows(P, model);
+        K.vec = vector_rows(P, model) && ((reinterpret_cast<uintptr_t>(K.err) |
+                                           reinterpret_cast<uintptr_t>(K.msk)) & 15) == 0;
         for (int s0 = 0; s0 < nsets; s0 += bt->wave) {
             const int cn = std::min(bt->wave, nsets - s0);
             P.set0 = K.set0 = s0;

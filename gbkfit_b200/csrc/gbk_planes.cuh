@@ -31,7 +31,7 @@ constexpr int KP_MAX_W = 384;         // longest window: 24 row groups, 12 chunk
 
 struct PlaneArgs {
     int Nx, Ny, Nz, Wx, Wy, nch, pitch;    // pitch: of the planes (floats)
-    int vec;                               // as BatchKernelArgs::vec
+    int vec;                               // Nx % 4 == 0, data and model on 16 bytes: float4 rows
     int hxp, ngw, set0;                    // padded spectrum columns; window row groups
     const float* mplanes;                  // (sets, Nz, Wy, pitch)
     const int* xrt;                        // (sets, Nz, Wy, nch)
@@ -41,7 +41,8 @@ struct PlaneArgs {
     // spec: (hxp / 16, Py, 16), of the PSF image shifted so that the crop starts
     // at the origin, scaled by 1 / (Px Py)
     const float2 *twx, *twy, *spec;
-    const float *obs, *iw;
+    const float *obs, *err, *msk;          // err, msk: may be null
+    float weight;
     float* model;                          // optional (nsets, Nz, Ny, Nx)
     double* partials;                      // (nsets, Nz, ceil(Ny / 16))
 };
@@ -200,8 +201,9 @@ __global__ void __launch_bounds__(KP_L * (N1 > 16 ? N1 : 16)) kp_cols(PlaneArgs 
 }
 
 // Crop rows [16 g, 16 g + 16) of a plane: the inverse of kp_rows (Z = X1 + i X2,
-// conj X1 + i conj X2 beyond n / 2), the first Nx columns, r = (m - d) iw
-// (objective.hpp:7-31) and the block's sum of r^2.
+// conj X1 + i conj X2 beyond n / 2), the first Nx columns, the residual
+// (objective.hpp:7-31) and the block's sum of r^2.  Error and mask are read here,
+// with the reference's division, so that a call meets them as they are.
 template<int N1>
 __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
 {
@@ -262,27 +264,37 @@ __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
         }
         __syncthreads();
     }
+    auto residual = [&](float m, float o, float e, float k) {
+        float r = m - o;
+        if (P.err) r /= e;
+        if (P.msk) r *= k;
+        return r * P.weight;
+    };
     for (int lr = p; lr < rows; lr += T / KP_L) {
         const float* ms = reinterpret_cast<const float*>(sm) + lr * n;
-        const float* od = P.obs + v0 + (long long)lr * P.Nx;
-        const float* iw = P.iw + v0 + (long long)lr * P.Nx;
+        const long long v = v0 + (long long)lr * P.Nx;
+        const float* od = P.obs + v;
+        const float* ed = P.err ? P.err + v : nullptr;
+        const float* kd = P.msk ? P.msk + v : nullptr;
         float* md = model ? model + (long long)lr * P.Nx : nullptr;
         if (P.vec) {
             // the rows start on 16 bytes
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int x = 4 * c; x < P.Nx; x += 4 * KP_L) {
                 const float4 o = __ldg(reinterpret_cast<const float4*>(od + x));
-                const float4 w = __ldg(reinterpret_cast<const float4*>(iw + x));
-                const float4 m = empty ? make_float4(0.f, 0.f, 0.f, 0.f)
-                                       : *reinterpret_cast<const float4*>(ms + x);
-                const float r0 = (m.x - o.x) * w.x, r1 = (m.y - o.y) * w.y;
-                const float r2 = (m.z - o.z) * w.z, r3 = (m.w - o.w) * w.w;
+                const float4 e = ed ? __ldg(reinterpret_cast<const float4*>(ed + x)) : zero;
+                const float4 k = kd ? __ldg(reinterpret_cast<const float4*>(kd + x)) : zero;
+                const float4 m = empty ? zero : *reinterpret_cast<const float4*>(ms + x);
+                const float r0 = residual(m.x, o.x, e.x, k.x), r1 = residual(m.y, o.y, e.y, k.y);
+                const float r2 = residual(m.z, o.z, e.z, k.z), r3 = residual(m.w, o.w, e.w, k.w);
                 sum += (r0 * r0 + r1 * r1) + (r2 * r2 + r3 * r3);
                 if (md) *reinterpret_cast<float4*>(md + x) = m;
             }
         } else {
             for (int x = c; x < P.Nx; x += KP_L) {
                 const float m = empty ? 0.f : ms[x];
-                const float r = (m - __ldg(od + x)) * __ldg(iw + x);
+                const float r = residual(m, __ldg(od + x), ed ? __ldg(ed + x) : 0.f,
+                                         kd ? __ldg(kd + x) : 0.f);
                 sum += r * r;
                 if (md) md[x] = m;
             }

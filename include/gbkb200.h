@@ -359,7 +359,9 @@ typedef struct {
     const double* lsf;      /* host: kernel_size[2] LSF, centred */
     const float* obs_d;     /* device: data (nz, ny, nx) */
     const float* obs_e;     /* device: errors, or NULL */
-    const float* obs_m;     /* device: mask, or NULL */
+    const float* obs_m;     /* device: mask, or NULL.  The FFT mode reads the three at
+                             * every call; the direct mode also makes tables of them at
+                             * creation, so that they must not change after it */
     float weight;
     int max_sets;           /* largest nsets of an evaluate call */
     int chunk;              /* sets per pipeline wave (0 = automatic: 256 MB of scratch, >= 8) */
