@@ -424,15 +424,14 @@ static KaFn ka_fn(int Kz)
     return t[Kz / 2];
 }
 
-static KaFn ka_t_fn(int Kz, bool sl)
+static KaFn ka_t_fn(int Kz, int lf)
 {
-    static KaFn t[2][KA_KMAX / 2 + 1] = {};
+    static KaFn t[3][KA_KMAX / 2 + 1] = {};
     static std::once_flag once;
     std::call_once(once, [] {
-        ka_t_register(t[0], false);
-        ka_t_register(t[1], true);
+        for (int f : {LINE_EX2, LINE_SCALED, LINE_EXP}) ka_t_register(t[f], f);
     });
-    return t[sl][Kz / 2];
+    return t[lf][Kz / 2];
 }
 
 // The model kernel of a model_variant (0-4; 0-3 named forms with identical
@@ -442,7 +441,7 @@ static KaFn ka_t_fn(int Kz, bool sl)
 static void pick_ka(gbkb200_batch* bt, int variant, bool tiles)
 {
     bt->ka_tiles = tiles;
-    bt->ka = tiles ? ka_t_fn(bt->P.Kz, variant == 4) : ka_fn(bt->P.Kz);
+    bt->ka = tiles ? ka_t_fn(bt->P.Kz, variant == 4 ? LINE_SCALED : LINE_EX2) : ka_fn(bt->P.Kz);
 }
 
 // the float4 rows of the residual (BatchKernelArgs::vec)
@@ -652,8 +651,8 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     P.nwfast = nodewise(d) ? 1 : 0;
     for (int t = 0; t < 33; ++t)
         P.lsfr[t] = t < Kz ? (float)d->lsf[d->kernel_size[2] - 1 - tz - t] : 0.f;
-    const int mv = d->model_variant < 0 || d->model_variant > 4 ? 3 : d->model_variant;
-    pick_ka(bt, mv, (long long)P.Nz * 16 <= 32 * 1024);
+    bt->ka_tiles = true;        // at most 880 planes (smem_z): 14 KB of range entries
+    bt->ka = ka_t_fn(P.Kz, LINE_EXP);
     PlaneArgs& K = bt->K;
     const int px = bt->pr.n, hx = px / 2 + 1, n = bt->pc.n;
     K.Nx = P.Nx; K.Ny = P.Ny; K.Nz = P.Nz; K.Wx = P.Wx; K.Wy = P.Wy;

@@ -245,6 +245,13 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf(B
     if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
 }
 
+// The line's profile in ka_lines_lsf_t
+enum {
+    LINE_EX2,       // amp 2^(-d^2 rinv) by ex2.approx, as ka_lines_lsf
+    LINE_SCALED,    // 2^(-t^2), t one multiply-add per channel
+    LINE_EXP        // orv (amp expf(-d^2 / (2 sigma^2))), as the drop-in thin disk and K1
+};
+
 // KA on compact spaxel tiles: a block per (set, 4 window rows, 32-column
 // chunk), its warp w on the 4 x 8 tile of columns [32 chunk + 8 w, + 8); lane
 // l takes spaxel (32 chunk + 8 w + (l & 7), 4 rg + (l >> 3)).  The lines of
@@ -261,16 +268,20 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 8 : 4)) ka_lines_lsf(B
 // instructions per group instead of a ballot and its bookkeeping per plane.
 // The lines, the LSF FIR and its order of operations are those of
 // ka_lines_lsf (identical values).
-// SL (scaled line): the exponent as -t^2 with t = zf (dz s) + (z0 - v) s and
+// LINE_SCALED: the exponent as -t^2 with t = zf (dz s) + (z0 - v) s and
 // s = sqrt(log2(e) / (2 sigma^2)), one multiply-add and one multiply per
 // channel instead of a multiply-add, an add and two multiplies; the same line
 // up to fp32 rounding (not bit-identical to the other forms).
+// LINE_EXP, for the plane-wise FFT mode: ex2.approx is 3.4e-8 low on average, which
+// the transforms' rounding does not hide; 130 us instead of 105 for the lines and the
+// LSF of 64 sets of 128 x 128 x 96 (eight blocks a SM; six and ten 134 and 132).
 // Ten blocks a SM (48 registers, 36 bytes spilled before the channel loop): 512
 // sets of 128 x 128 x 96 in 472 us, 490 with eight and 64 registers, 473 with
 // nine, 480 with twelve; at 15 taps 67.5, 68.2, 71.4 and 70.6 us (16 sets of 256 x
 // 240 x 128).
-template<int KZ, bool SL>
-__global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 10 : 4)) ka_lines_lsf_t(BatchKernelArgs P, int* status)
+template<int KZ, int LF>
+__global__ void __launch_bounds__(KA_THREADS, (KZ > 15 ? 4 : LF == LINE_EXP ? 8 : 10))
+ka_lines_lsf_t(BatchKernelArgs P, int* status)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rg = blockIdx.x / P.nch, chunk = blockIdx.x % P.nch;   // grid: ceil(Wy / 4) nch
@@ -285,23 +296,31 @@ __global__ void __launch_bounds__(KA_THREADS, (KZ <= 15 ? 10 : 4)) ka_lines_lsf_
     int bad = 0;
     SpaxelOut o{};
     int lo = INT_MAX, hi = -1;
-    float amp = 0.f, rinv = 0.f;
+    float amp = 0.f, rinv = LF == LINE_EXP ? 1.f : 0.f;
     const bool on = row_ok && x < P.Wx &&
                     (P.nwfast ? smdisk_spaxel_nw(a, kc, x, y, o) : smdisk_spaxel(a, kc, x, y, 0, o, bad));
     if (on && line_window(o.vv, o.dv, P.Wz, a.spec_step, a.spec_zero, lo, hi)) {
-        amp = o.orv * (1 / (o.dv * sqrtf(2 * GBK_PI)));
-        rinv = 1.4426950408889634f / (2 * o.dv * o.dv);
+        amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
+        if (LF == LINE_EXP) {
+            rinv = 2 * o.dv * o.dv;             // the divisor
+        } else {
+            amp = o.orv * amp;
+            rinv = 1.4426950408889634f / (2 * o.dv * o.dv);
+        }
     } else {
         lo = INT_MAX;
         hi = -1;
     }
     const float v = o.vv, z0 = a.spec_zero, dz = a.spec_step;
     const unsigned wlen = (unsigned)hi - (unsigned)lo;
-    const float sc = SL ? sqrtf(rinv) : 0.f;
+    const float sc = LF == LINE_SCALED ? sqrtf(rinv) : 0.f;
     const float dzs = dz * sc, cs = (z0 - v) * sc;
     auto line_f = [&](int z, float zf) {
         float e;
-        if constexpr (SL) {
+        if constexpr (LF == LINE_EXP) {
+            const float d = (z0 + zf * dz) - v;
+            return (unsigned)z - (unsigned)lo <= wlen ? o.orv * (amp * expf(-d * d / rinv)) : 0.f;
+        } else if constexpr (LF == LINE_SCALED) {
             const float t = fmaf(zf, dzs, cs);
             asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-(t * t)));
         } else {
@@ -838,7 +857,7 @@ static_assert(KA_KMAX <= 33 && KB_KMAX <= 33, "coefficient arrays of BatchKernel
 void ka_register_short(KaFn* t);
 void ka_register_long(KaFn* t);
 // t[Kz / 2]: the model kernel on 4 x 8 spaxel tiles (ka_lines_lsf_t)
-void ka_t_register(KaFn* t, bool sl);
+void ka_t_register(KaFn* t, int lf);
 // t[Kz / 2]: the LSF FIR of given model cubes
 typedef void (*KcFn)(BatchKernelArgs, const float*);
 void kc_register(KcFn* t);

@@ -12,9 +12,13 @@
 // The 3-D form (K1-K5 of batched.cu) transforms z as well, for an LSF of
 // ten-odd taps: two more passes over a cube that left the L2, and run-time
 // radices throughout.  64 sets of 128 x 128 x 96 with a Moffat PSF in waves of
-// 16: 6420 us in the 3-D form, 850 us here (model and LSF 104, rows 153, columns
-// 345, residual 245), bound by instruction issue (65-70 % of cycles, about 75
-// instructions per spectrum value and pass).  Lines of 16 N1 points, so that a
+// 16: 6420 us in the 3-D form, 920 us here (model and LSF 130, rows 153, columns
+// 345, residual 275), bound by instruction issue (65-70 % of cycles, about 75
+// instructions per spectrum value and pass).  The lines and the residual are
+// those of the 3-D form, operation by operation, and r^2 is summed in fp64 (with
+// ex2.approx lines and a residual weight made at creation 865 us, and chi^2 1.79e-7
+// from its 64-bit value over 48 drawn batches, now 1.48e-7, the 3-D form 1.55e-7).
+// Lines of 16 N1 points, so that a
 // thread's elements lie 16 rows or columns apart and masks, addresses and zero
 // row groups fold into compile-time offsets (with other factors the columns
 // took 366-434 us), and two real rows per transform instead of the even/odd
@@ -203,21 +207,22 @@ __global__ void __launch_bounds__(KP_L * (N1 > 16 ? N1 : 16)) kp_cols(PlaneArgs 
 // Crop rows [16 g, 16 g + 16) of a plane: the inverse of kp_rows (Z = X1 + i X2,
 // conj X1 + i conj X2 beyond n / 2), the first Nx columns, the residual
 // (objective.hpp:7-31) and the block's sum of r^2.  Error and mask are read here,
-// with the reference's division, so that a call meets them as they are.
+// with the reference's division, so that a call meets them as they are (ten
+// instructions per voxel more than a weight made once: 245 -> 272 us).
 template<int N1>
 __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
 {
     constexpr int N2 = 16, n = N1 * N2, T = kp_threads(N1), P2 = N2 + 1;
     extern __shared__ float2 sm[];          // 8 pairs of N1 P2, then n twiddles
     float2* s_tw = sm + KP_P * N1 * P2;
-    __shared__ float s_part[T / 32];
+    __shared__ double s_part[T / 32];
     const int zo = blockIdx.y, y0 = blockIdx.x * KP_L, rows = min(KP_L, P.Ny - y0);
     const long long plane = (long long)blockIdx.z * P.Nz + zo;
     const int b = P.set0 + blockIdx.z;
     const long long v0 = ((long long)zo * P.Ny + y0) * P.Nx;       // the rows in the data cube
     float* model = P.model ? P.model + (long long)b * P.Nz * P.Ny * P.Nx + v0 : nullptr;
     const int p = threadIdx.x / KP_L, c = threadIdx.x % KP_L;
-    float sum = 0.f;
+    double sum = 0.0;
     const bool empty = plane_groups(P, plane) == 0u;
     if (!empty) {
         for (int i = threadIdx.x; i < n; i += T) s_tw[i] = P.twx[i];
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
                 const float4 m = empty ? zero : *reinterpret_cast<const float4*>(ms + x);
                 const float r0 = residual(m.x, o.x, e.x, k.x), r1 = residual(m.y, o.y, e.y, k.y);
                 const float r2 = residual(m.z, o.z, e.z, k.z), r3 = residual(m.w, o.w, e.w, k.w);
-                sum += (r0 * r0 + r1 * r1) + (r2 * r2 + r3 * r3);
+                sum += (double)((r0 * r0 + r1 * r1) + (r2 * r2 + r3 * r3));
                 if (md) *reinterpret_cast<float4*>(md + x) = m;
             }
         } else {
@@ -295,7 +300,7 @@ __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
                 const float m = empty ? 0.f : ms[x];
                 const float r = residual(m, __ldg(od + x), ed ? __ldg(ed + x) : 0.f,
                                          kd ? __ldg(kd + x) : 0.f);
-                sum += r * r;
+                sum += (double)(r * r);
                 if (md) md[x] = m;
             }
         }
@@ -305,9 +310,9 @@ __global__ void __launch_bounds__(kp_threads(N1)) kp_resid(PlaneArgs P)
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float s = 0.f;
+        double s = 0.0;
         for (int w = 0; w < T / 32; ++w) s += s_part[w];
-        P.partials[((long long)b * P.Nz + zo) * gridDim.x + blockIdx.x] = (double)s;
+        P.partials[((long long)b * P.Nz + zo) * gridDim.x + blockIdx.x] = s;
     }
 }
 
