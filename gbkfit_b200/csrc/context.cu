@@ -171,7 +171,7 @@ std::map<std::pair<int, const void*>, SmemLimit> g_smem_limits;   // by (device,
 
 int gbk_raise_smem_limit(const void* fn, size_t bytes)
 {
-    if (bytes <= 32 * 1024) return GBKB200_OK;      // the kernels' static arrays take up to 10 KB
+    if (bytes <= 32 * 1024) return GBKB200_OK;      // the kernels' static arrays take up to 12 KB
     int dev = 0;
     GBK_CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(g_smem_mutex);

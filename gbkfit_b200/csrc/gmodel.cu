@@ -80,23 +80,14 @@ __global__ void __launch_bounds__(32 * THIN_Y) smdisk_thin_kernel(DiskArgs a, in
     if (bad) atomicOr(status, GBK_STATUS_BAD_TRAIT);
 }
 
-// A line at distance d from its centre without the amplitude:
-// exp(-d^2 / (2 sigma^2)) as 2^(-d^2 rinv) with rinv = log2(e) / (2 sigma^2),
-// by the PTX ex2.approx instruction (relative error ~2^-22; inside the +-5
-// sigma window the argument is >= -18.1, far from the flush to zero)
-__device__ __forceinline__ float line_e2(float d, float rinv)
-{
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-(d * d) * rinv));
-    return e;
-}
-
 // Thick disk (or thin with spatial z > 1): block (32, 16) owns 32 adjacent
 // spaxel columns of one row.  Its warps evaluate sixteen spatial z at a time and
 // put their lines' parameters into shared memory; then warp w adds, for every
 // line of the round, the channels w, w + 16, ... of the columns, each channel of
 // a column having one owner: no atomics, and sums in a fixed order (shared
-// fp32 atomics took 145 us for a 96 x 96 x 96 grid with 96 channels, this 59).
+// fp32 atomics took 145 us for a 96 x 96 x 96 grid with 96 channels, this 66).
+// The lines are the thin disk's, operation by operation (ex2.approx: 59 us, but
+// 3.4e-8 low on average).
 // With USE_SMEM the spectral columns (spec_size x 32) are accumulated in shared
 // memory and added to the cube at the end; else (spectra too long) in the cube.
 constexpr int TH = 16;          // warps: a power of two
@@ -104,7 +95,7 @@ template<bool USE_SMEM>
 __global__ void __launch_bounds__(32 * TH) smdisk_thick_kernel(DiskArgs a, int* status)
 {
     extern __shared__ float tile[];
-    __shared__ float s_v[TH][32], s_amp[TH][32], s_rinv[TH][32];
+    __shared__ float s_v[TH][32], s_orv[TH][32], s_amp[TH][32], s_2s2[TH][32];
     __shared__ int s_lo[TH][32], s_hi[TH][32];
     const int tx = threadIdx.x, tz = threadIdx.y;
     const int x = blockIdx.x * 32 + tx;
@@ -119,15 +110,16 @@ __global__ void __launch_bounds__(32 * TH) smdisk_thick_kernel(DiskArgs a, int* 
         const int z = z0 + tz;
         SpaxelOut o;
         int zlo = 0, zhi = -1;
-        float amp = 0.f, rinv = 0.f, v = 0.f;
+        float amp = 0.f, inv2c2 = 0.f, v = 0.f, orv = 0.f;
         if (x < a.sx && z < a.sz && smdisk_spaxel(a, kc, x, y, z, o, bad)) {
             if (a.image) atomicAdd(&a.image[x + (long long)a.sx * y], o.orv);
             smdisk_side_outputs(a, x, y, z, o);
             if (a.scube &&
                 line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
-                amp = o.orv * (1 / (o.dv * sqrtf(2 * GBK_PI)));
-                rinv = 0.7213475204444817f / (o.dv * o.dv);
+                amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
+                inv2c2 = 2 * o.dv * o.dv;
                 v = o.vv;
+                orv = o.orv;
             } else {
                 zlo = 0;
                 zhi = -1;
@@ -135,18 +127,19 @@ __global__ void __launch_bounds__(32 * TH) smdisk_thick_kernel(DiskArgs a, int* 
         }
         if (!a.scube) continue;             // every thread
         s_v[tz][tx] = v;
+        s_orv[tz][tx] = orv;
         s_amp[tz][tx] = amp;
-        s_rinv[tz][tx] = rinv;
+        s_2s2[tz][tx] = inv2c2;
         s_lo[tz][tx] = zlo;
         s_hi[tz][tx] = zhi;
         __syncthreads();
         for (int k = 0; k < TH; ++k) {
             const int lo = s_lo[k][tx], hi = s_hi[k][tx];
-            const float vk = s_v[k][tx], ak = s_amp[k][tx], ik = s_rinv[k][tx];
+            const float vk = s_v[k][tx], ok = s_orv[k][tx], ak = s_amp[k][tx], ck = s_2s2[k][tx];
             // the first channel >= lo that is tz modulo TH
             for (int zs = lo + ((tz - lo) & (TH - 1)); zs <= hi; zs += TH) {
                 const float d = (a.spec_zero + zs * a.spec_step) - vk;
-                const float f = ak * line_e2(d, ik);
+                const float f = ok * (ak * expf(-d * d / ck));
                 if (USE_SMEM) tile[zs * 32 + tx] += f;
                 else col[plane * zs] += f;
             }
@@ -164,6 +157,17 @@ __global__ void __launch_bounds__(32 * TH) smdisk_thick_kernel(DiskArgs a, int* 
 }
 
 // ---- mcdisk ------------------------------------------------------------------
+
+// The cloud's line at distance d from its centre without the amplitude:
+// exp(-d^2 / (2 sigma^2)) as 2^(-d^2 rinv) with rinv = log2(e) / (2 sigma^2),
+// by the PTX ex2.approx instruction (relative error ~2^-22; inside the +-5
+// sigma window the argument is >= -18.1, far from the flush to zero)
+__device__ __forceinline__ float line_e2(float d, float rinv)
+{
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-(d * d) * rinv));
+    return e;
+}
 
 // Philox-4x32-10 (Salmon et al., SC'11), counter {ci, k/4, 0, 0}, key = seed
 struct Philox {

@@ -22,8 +22,8 @@ def _thick():
     from tests.test_gpu_disk_kernels import _disk, _geo
     disk, p = _disk(True)
     gm = DriverB200(0).backends().gmodel(np.float32)
-    # 128 bytes a channel beside 10 KB: exactly 48 KB at 304
-    for spec in (304, 305, 320, 352, 384):
+    # 128 bytes a channel beside 12 KB: exactly 48 KB at 288
+    for spec in (288, 289, 320, 352, 384):
         geo, packed = _geo(20, 3, 9, spec), disk.pack(p)
         cube = torch.zeros((spec, 3, 20), device='cuda')
         gpu_smdisk(gm, upload(packed, 'cuda'), geo, dict(scube=cube))
