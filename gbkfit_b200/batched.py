@@ -198,6 +198,8 @@ class BatchedSMDisk:
                                       ctypes.byref(cm)), 'batch_info')
         self.fft_size, self.chunk, self.work_bytes = tuple(fs), ch.value, wb.value
         self.conv_mode = {1: 'fft', 2: 'direct'}[cm.value]
+        # the FFT mode's plane-wise form (fft_size: its line lengths and 1)
+        self.planewise = bool(_lib.gbkb200_batch_planewise(h))
         self.psf_rank = rank
         self.chi2 = torch.zeros(self.max_sets, device=dev)
         self._graph = None
@@ -508,8 +510,7 @@ class BatchedSMDisk:
         ms = (ctypes.c_double * 6)()
         n = (c_int * 6)()
         check(_lib.gbkb200_batch_timing(self.handle, ms, n), 'batch_timing')
-        planes = _lib.gbkb200_batch_planewise(self.handle)
-        names = STAGE_KERNELS['planes' if planes else self.conv_mode]
+        names = STAGE_KERNELS['planes' if self.planewise else self.conv_mode]
         return {names[i]: (ms[i], n[i]) for i in range(6) if n[i]}
 
     def work_counters(self):

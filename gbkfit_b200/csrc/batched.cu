@@ -659,10 +659,11 @@ static int setup_planes(gbkb200_batch* bt, const gbkb200_batch_desc* d)
     K.nch = P.nch; K.pitch = P.pitch;
     K.hxp = (hx + KP_L - 1) / KP_L * KP_L;
     K.ngw = (P.Wy + KP_L - 1) / KP_L;
-    // sets per sub-wave: at most 256 MB of spectra.  Keeping them in L2 does
-    // not pay (64 sets of 128 x 128 x 96, spectra of 24 / 48 / 100 / 220 MB per
-    // sub-wave: 1381 / 1107 / 1008 / 972 us; the passes are bound by issue and
-    // small launches leave the chip idle); beyond that only memory grows
+    // sets per sub-wave: at most 256 MB of row spectra (their crop rows and the
+    // planes take up to as much again, each).  Keeping them in L2 does not pay
+    // (64 sets of 128 x 128 x 96, spectra of 26 / 51 / 102 / 205 MB per sub-wave:
+    // 1716 / 1263 / 1051 / 925 us; the passes are bound by issue and small
+    // launches leave the chip idle); beyond that only memory grows
     const size_t per_set = (size_t)P.Nz * K.ngw * KP_L * K.hxp * sizeof(float2);
     if (d->chunk <= 0) bt->chunk = auto_chunk(bt, per_set);
     bt->wave = (int)std::max<size_t>(1, std::min<size_t>(bt->chunk, (256u << 20) / per_set));
@@ -909,6 +910,10 @@ extern "C" int gbkb200_batch_create(gbkb200_ctx* ctx, const gbkb200_batch_desc* 
         rc = setup_planes(bt, d);
         if (rc == GBKB200_OK) {
             GBK_CUDA_TRY(cudaGetLastError());
+            for (float2*& tw : bt->tw) {        // of the 3-D grid
+                cudaFree(tw);
+                tw = nullptr;
+            }
             *out = bt;
             return GBKB200_OK;
         }
@@ -999,9 +1004,11 @@ extern "C" int gbkb200_batch_info(const gbkb200_batch* bt, int fft_size[3], int*
     if (!bt) return GBKB200_ERR_INVALID_ARG;
     if (conv_mode) *conv_mode = bt->direct ? 2 : 1;
     if (fft_size) {
-        fft_size[0] = bt->P.Px; fft_size[1] = bt->P.Py; fft_size[2] = bt->P.Pz;
+        fft_size[0] = bt->planes ? bt->pr.n : bt->P.Px;
+        fft_size[1] = bt->planes ? bt->pc.n : bt->P.Py;
+        fft_size[2] = bt->planes ? 1 : bt->P.Pz;
     }
-    if (chunk) *chunk = bt->chunk;
+    if (chunk) *chunk = bt->planes ? bt->wave : bt->chunk;
     if (work_bytes) {
         // device bytes the evaluator holds (its scratch, tables and partials)
         const BatchKernelArgs& P = bt->P;

@@ -342,7 +342,8 @@ typedef struct gbkb200_batch gbkb200_batch;
 typedef struct {
     int size[3];            /* data cube (nx, ny, nz) */
     int kernel_size[3];     /* PSF box (x, y) and LSF box (z), odd */
-    int fft_size[3];        /* FFT grid >= size + kernel_size - 1; 0 = automatic */
+    int fft_size[3];        /* FFT grid >= size + kernel_size - 1; 0 = automatic (the plane-wise
+                             * FFT mode takes its own line lengths) */
     float spat_step[2];     /* evaluation grid step (x, y) */
     float spat_zero[2];     /* evaluation grid zero (DCube scratch zero, x, y) */
     float spec_step;
@@ -364,9 +365,13 @@ typedef struct {
                              * creation, so that they must not change after it */
     float weight;
     int max_sets;           /* largest nsets of an evaluate call */
-    int chunk;              /* sets per pipeline wave (0 = automatic: 256 MB of scratch, >= 8) */
-    int rows_k1;            /* spectral rows per shared-memory group of the model kernel (0 = 16) */
-    int rows_k5;            /* rows per block of the residual kernel (0 = 8) */
+    int chunk;              /* sets per pipeline wave (0 = automatic: up to 256 MB of planes in the
+                             * direct mode, >= 8 sets; of row spectra in the plane-wise FFT
+                             * mode, whose crop rows and planes take up to as much again,
+                             * each, and which divides a larger chunk; 8 in the 3-D form) */
+    int rows_k1;            /* 3-D form: spectral rows per shared-memory group of the model
+                             * kernel (0 = 16) */
+    int rows_k5;            /* 3-D form: rows per block of the residual kernel (0 = 8) */
     int conv_mode;          /* 0 = automatic, 1 = FFT, 2 = direct separable FIR */
     int psf_rank;           /* direct mode: PSF = sum_r u_r(y) v_r(x), rank <= 8 */
     const double* psf_u;    /* host: (psf_rank, kernel_size[1]) */
@@ -419,9 +424,9 @@ int gbkb200_batch_query(const gbkb200_batch* b, int* done);
  * word its kernels raised (GBKB200_ERR_BAD_TRAIT: a model of the submission
  * met an unknown trait uid), which is then cleared */
 int gbkb200_batch_take_status(gbkb200_batch* b);
-/* the chosen FFT grid, chunk, the device bytes the evaluator holds (its
- * work space, tables and partials) and the convolution mode (1 = FFT,
- * 2 = direct) */
+/* the chosen FFT grid (plane-wise: the x and y line lengths and 1), the sets of a
+ * wave, the device bytes the evaluator holds (its work space, tables and
+ * partials) and the convolution mode (1 = FFT, 2 = direct) */
 int gbkb200_batch_info(const gbkb200_batch* b, int fft_size[3], int* chunk, size_t* work_bytes,
                        int* conv_mode);
 /* 1 where the FFT mode convolves plane by plane (2-D transforms after the
