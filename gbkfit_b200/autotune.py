@@ -3,7 +3,7 @@
 Knobs (all change speed only, never results beyond fp32 rounding):
 * ``conv``: direct separable FIR (low-rank PSFs) or FFT convolution;
 * ``fft_size``: FFT grid per axis, any 2/3/5/7-smooth size >= the window
-  (x even);
+  (x even); not in the plane-wise form, which takes its own line lengths;
 * ``chunk``: parameter sets per pipeline wave (the wave's intermediates
   should stay in L2);
 * ``band``: output rows per PSF block of the direct mode (smaller bands: more
@@ -11,7 +11,8 @@ Knobs (all change speed only, never results beyond fp32 rounding):
 * ``model_variant``: the direct mode's model kernel (3: a 4 x 8 spaxel tile
   per warp; 4: the same with the line exponent from one multiply-add, the same
   values up to fp32 rounding);
-* ``rows_k1``: spectral rows per shared-memory group of the model kernel.
+* ``rows_k1``: spectral rows per shared-memory group of the model kernel (3-D
+  FFT form).
 
 Coordinate descent from the defaults; every trial builds an evaluator and
 times a few full evaluations with CUDA events.  Results are cached per
@@ -69,13 +70,17 @@ def _store(key, cfg):
         pass
 
 
-def time_config(w, data, err, nsets, cfg, reps=3):
+def time_config(w, data, err, nsets, cfg, reps=3, info=None):
+    """Median milliseconds of an evaluation (inf where cfg is refused); info
+    receives whether the evaluator is of the plane-wise form."""
     import torch
     from .batched import BatchedSMDisk
     try:
         ev = BatchedSMDisk(w.disk, w.geom, data, err, max_sets=nsets, **cfg)
     except RuntimeError:
         return float('inf')
+    if info is not None:
+        info['planewise'] = ev.planewise
     bufs = ev.alloc_inputs(nsets)
     ev.upload(ev.pack(w.params, nsets), bufs, nsets)
     ev.evaluate_device(bufs, nsets)
@@ -105,9 +110,10 @@ def tune_batched(w, data, err, nsets, budget_s=60.0, use_cache=True):
     t_end = time.time() + budget_s
     # direct separable convolution (when the PSF is rank 1): chunk, then band
     best_d, best_dt = None, float('inf')
+    tiles = g.size[2] * 16 <= 32 * 1024        # the tile model kernel's cubes
     for chunk in (32, 64, 128, 256, 512):
         cfg = dict(fft_size=(0, 0, 0), chunk=chunk, rows_k1=16, conv='direct', band=0,
-                   model_variant=0)
+                   model_variant=3 if tiles else 0)
         t = time_config(w, data, err, nsets, cfg)
         if t < best_dt:
             best_d, best_dt = cfg, t
@@ -119,10 +125,8 @@ def tune_batched(w, data, err, nsets, budget_s=60.0, use_cache=True):
             t = time_config(w, data, err, nsets, cfg)
             if t < best_dt:
                 best_d, best_dt = cfg, t
-        # the model kernel's variants
-        base = dict(best_d)
-        for mv in (3, 4):
-            cfg = dict(base, model_variant=mv)
+        if tiles:
+            cfg = dict(best_d, model_variant=4)
             t = time_config(w, data, err, nsets, cfg)
             if t < best_dt:
                 best_d, best_dt = cfg, t
@@ -130,11 +134,14 @@ def tune_batched(w, data, err, nsets, budget_s=60.0, use_cache=True):
     cand = [smooth_sizes(win[0], even=True), smooth_sizes(win[1]), smooth_sizes(win[2])]
     best = dict(fft_size=(cand[0][0], cand[1][0], cand[2][0]), chunk=8, rows_k1=16, conv='fft',
                 band=0)
-    best_t = time_config(w, data, err, nsets, best)
+    info = {}
+    best_t = time_config(w, data, err, nsets, best, info=info)
     trials = []
-    for knob, values in (('chunk', (2, 4, 8, 16, 32)), ('rows_k1', (8, 16, 32)),
-                         ('fft_x', cand[0]), ('fft_y', cand[1]), ('fft_z', cand[2]),
-                         ('chunk', (2, 4, 8, 16, 32))):
+    knobs = [('chunk', (2, 4, 8, 16, 32))]
+    if not info.get('planewise'):
+        knobs += [('rows_k1', (8, 16, 32)), ('fft_x', cand[0]), ('fft_y', cand[1]),
+                  ('fft_z', cand[2]), ('chunk', (2, 4, 8, 16, 32))]
+    for knob, values in knobs:
         for v in values:
             if time.time() > t_end:
                 break

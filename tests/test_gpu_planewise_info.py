@@ -1,4 +1,5 @@
-"""What an evaluator of the plane-wise FFT mode says about itself."""
+"""What an evaluator of the plane-wise FFT mode says about itself, and what the
+tuner tries on it."""
 
 import numpy as np
 import pytest
@@ -35,3 +36,19 @@ def test_info(gpu, nsets, chunk):
         nsets * 24 * -(-44 // 16) * 8
     assert ev.chunk * lines <= 256 << 20 and crop <= lines and 132 * rows <= ev.chunk * lines
     ev.close()
+
+
+def test_tuner_leaves_the_3d_knobs_alone(gpu, monkeypatch):
+    from gbkfit_b200 import autotune
+    w, data = _workload(6)
+    tried, orig = [], autotune.time_config
+
+    def time_config(w, data, err, nsets, cfg, *a, **kw):
+        if cfg['conv'] == 'fft':
+            tried.append(cfg)
+        return orig(w, data, err, nsets, cfg, *a, **kw)
+
+    monkeypatch.setattr(autotune, 'time_config', time_config)
+    autotune.tune_batched(w, data, None, 6, use_cache=False)
+    assert len(tried) > 1 and len({(c['fft_size'], c['rows_k1']) for c in tried}) == 1
+    assert len({c['chunk'] for c in tried}) == len(tried)
