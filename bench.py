@@ -264,8 +264,8 @@ def parity_sample(ev, w, bufs, nsets, data, err, sets=(0, 255, 511)):
 
 
 def autotune(w, data, err, nsets, budget_s=60.0):
-    """Time candidate pipeline shapes (chunk, rows per K1 group, FFT grid);
-    returns the fastest configuration."""
+    """Time candidate pipeline shapes (gbkfit_b200/autotune.py); returns the fastest
+    configuration."""
     import torch
     from gbkfit_b200.autotune import tune_batched
     return tune_batched(w, data, err, nsets, budget_s=budget_s)
@@ -401,7 +401,9 @@ def run_b200(args):
     out = None
     if rank == 0:
         n_chunks = (nsets + ev.chunk - 1) // ev.chunk
-        per_chunk = 2 if ev.conv_mode == 'direct' else 5
+        # kernels per wave: model and PSF; model, rows, columns and
+        # residual; K1-K5
+        per_chunk = 2 if ev.conv_mode == 'direct' else 4 if ev.planewise else 5
         plain = plain_per_call(w, data, err) if args.plain else None
         serving = serving_run() if args.serving else None
         cpu = cpu_baseline(w, data, err) if args.cpu_baseline else None
@@ -945,11 +947,11 @@ def main():
                     help='force the convolution mode (default: tuned)')
     ap.add_argument('--chunk', type=int, default=0, help='force the sets per wave (default: tuned)')
     ap.add_argument('--psf-variant', type=int, default=-1, choices=[-1, 0, 1, 2, 3, 4, 5, 6, 7],
-                    help='PSF kernel variant of the direct mode (default: tuned)')
+                    help='accepted; one PSF kernel is left')
     ap.add_argument('--model-variant', type=int, default=-1, choices=[-1, 0, 1, 2, 3, 4],
-                    help='model kernel of the direct mode: 0 one chunk per warp, 1 chunk '
-                         'pairs, 2 4x8 spaxel tiles, 3 tiles with transposed range masks, '
-                         '4 as 3 with the scaled line exponent (default: tuned)')
+                    help='model kernel of the direct mode: 0-3 the 4x8 spaxel tiles (0 and 1 '
+                         'a 32-column chunk per warp above 2048 channels), 4 the tiles with '
+                         'the scaled line exponent (default: tuned)')
     ap.add_argument('--band', type=int, default=0,
                     help='force the output rows per PSF block of the direct mode (default: tuned)')
     ap.add_argument('--workload', default='smdisk_batch128',
