@@ -132,8 +132,8 @@ class SMDiskChi2:
         self.dev = torch.device('cuda', device)
         self.stream = torch.cuda.current_stream(self.dev)
         self.ctx = _native.Context(device=device, stream=self.stream, sync=False)
-        # the gradient is handed out in float64: it keeps the transforms (and
-        # so the rounding) that its results came from so far
+        # the gradient is handed out in float64: one family of transforms, so that its
+        # rounding is the same from build to build (include/gbkb200.h)
         self.ctx.set_fft(1)
         f32 = lambda a: None if a is None else torch.as_tensor(
             np.ascontiguousarray(a, np.float32)).to(self.dev)

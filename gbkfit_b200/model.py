@@ -553,7 +553,7 @@ class DModelMMaps:
             dc.prepare(driver, gmodel.has_weights())
             # the second moment weighs the cube's rounding by the squared
             # velocity: faint spaxels move by ~5e-5 with other transforms, so
-            # the maps keep the ones they came from so far
+            # the maps use one family of them (include/gbkb200.h)
             dc._backend_fft._ctx.set_fft(1)
             self._backend = driver.backends().dmodel(dc.dtype())
             n = len(self._orders)
