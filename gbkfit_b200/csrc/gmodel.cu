@@ -29,34 +29,33 @@ namespace gbk {
 // waited for the write before it), and blocks are two warps so that a small
 // plane spreads over the chip (96 x 96 x 96: 14 us, 21 us before).
 constexpr int THIN_Y = 2, THIN_Z = 8;
-__global__ void __launch_bounds__(32 * THIN_Y) smdisk_thin_kernel(DiskArgs a, int* status)
+__global__ void __launch_bounds__(32 * THIN_Y) smdisk_thin_kernel(DiskArgs a, int y0, int* status)
 {
     const int x = blockIdx.x * 32 + threadIdx.x;
+    const int y = y0 + blockIdx.y * THIN_Y + threadIdx.y;
+    const bool inside = x < a.sx && y < a.sy;
     int bad = 0;
     DiskConst kc = disk_const(a);
-    // one pass, but for more rows than a grid dimension holds pairs (whole warps)
-    for (int y = blockIdx.y * THIN_Y + threadIdx.y; y < a.sy; y += gridDim.y * THIN_Y) {
-        SpaxelOut o;
-        bool on = x < a.sx && smdisk_spaxel(a, kc, x, y, 0, o, bad);
-        int zlo = INT_MAX, zhi = -1;
-        float amp = 0, inv2c2 = 0;
-        if (on) {
-            if (a.image) a.image[x + (long long)a.sx * y] += o.orv;
-            smdisk_side_outputs(a, x, y, 0, o);
-            if (a.scube &&
-                line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
-                amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
-                inv2c2 = 2 * o.dv * o.dv;
-            } else {
-                zlo = INT_MAX;
-                zhi = -1;
-            }
+    SpaxelOut o;
+    bool on = inside && smdisk_spaxel(a, kc, x, y, 0, o, bad);
+    int zlo = INT_MAX, zhi = -1;
+    float amp = 0, inv2c2 = 0;
+    if (on) {
+        if (a.image) a.image[x + (long long)a.sx * y] += o.orv;
+        smdisk_side_outputs(a, x, y, 0, o);
+        if (a.scube && line_window(o.vv, o.dv, a.spec_size, a.spec_step, a.spec_zero, zlo, zhi)) {
+            amp = 1 / (o.dv * sqrtf(2 * GBK_PI));
+            inv2c2 = 2 * o.dv * o.dv;
+        } else {
+            zlo = INT_MAX;
+            zhi = -1;
         }
-        // channel loop over the union of the warp's windows: coalesced rows
-        const unsigned full = 0xffffffffu;
-        int wlo = __reduce_min_sync(full, zlo);
-        int whi = __reduce_max_sync(full, zhi);
-        if (!a.scube) continue;
+    }
+    // channel loop over the union of the warp's windows: coalesced rows
+    const unsigned full = 0xffffffffu;
+    int wlo = __reduce_min_sync(full, zlo);
+    int whi = __reduce_max_sync(full, zhi);
+    if (a.scube) {
         const long long plane = (long long)a.sx * a.sy;
         float* col = a.scube + (x + (long long)a.sx * y);
         for (int z0 = wlo; z0 <= whi; z0 += THIN_Z) {
@@ -871,9 +870,12 @@ int gbk_launch_smdisk(const DiskArgs& a, cudaStream_t stream, int* status)
 {
     const bool thin = a.rht.uids == nullptr;
     if (thin && a.sz == 1) {
-        dim3 block(32, THIN_Y),
-            grid((a.sx + 31) / 32, std::min((a.sy + THIN_Y - 1) / THIN_Y, 65535));
-        smdisk_thin_kernel<<<grid, block, 0, stream>>>(a, status);
+        // one launch, but for more rows than a grid dimension holds pairs
+        for (long long y0 = 0; y0 < a.sy; y0 += 65535 * THIN_Y) {
+            const long long pairs = (a.sy - y0 + THIN_Y - 1) / THIN_Y;
+            const dim3 grid((a.sx + 31) / 32, (unsigned)std::min<long long>(pairs, 65535));
+            smdisk_thin_kernel<<<grid, dim3(32, THIN_Y), 0, stream>>>(a, (int)y0, status);
+        }
     } else {
         dim3 block(32, TH), grid((a.sx + 31) / 32, a.sy);
         size_t smem = a.scube ? (size_t)a.spec_size * 32 * sizeof(float) : 0;
