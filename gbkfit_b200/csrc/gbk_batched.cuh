@@ -457,7 +457,7 @@ __device__ __forceinline__ void kb_zero_rows(float* m, int nx, bool vec, int r0,
 //     data.
 // The zero-model residual outside the box comes from the summed-area table.
 //
-// Bound by issue (59 % of cycles) and shared-memory wavefronts (63 %) with 16
+// Bound by issue (62 % of cycles) and shared-memory wavefronts (66 %) with 16
 // warps a SM; a block's phases (cycles, 512 sets of 128 x 128 x 96): box 3.0k, to
 // the loads 1.4k, loads 7.0k, x FIR 5.3k, y FIR 4.9k, residual 6.0k.  That batch:
 // 1282 us with run-time divisions in the loads and outside the box and

@@ -13,16 +13,15 @@
 // ten-odd taps: two more passes over a cube that left the L2, and run-time
 // radices throughout.  64 sets of 128 x 128 x 96 with a Moffat PSF in waves of
 // 16: 6420 us in the 3-D form, 920 us here (model and LSF 130, rows 153, columns
-// 345, residual 275), bound by instruction issue (65-70 % of cycles, about 75
+// 345, residual 275), bound by instruction issue (62-76 % of cycles, about 75
 // instructions per spectrum value and pass).  The lines and the residual are
 // those of the 3-D form, operation by operation, and r^2 is summed in fp64 (with
 // ex2.approx lines and a residual weight made at creation 865 us, and chi^2 1.79e-7
 // from its 64-bit value over 48 drawn batches, now 1.48e-7, the 3-D form 1.55e-7).
-// Lines of 16 N1 points, so that a
-// thread's elements lie 16 rows or columns apart and masks, addresses and zero
-// row groups fold into compile-time offsets (with other factors the columns
-// took 366-434 us), and two real rows per transform instead of the even/odd
-// split (rows and residual 209 and 299 us with it).
+// Lines of 16 N1 points, so that a thread's elements lie 16 rows or columns apart and
+// masks, addresses and zero row groups fold into compile-time offsets (with other
+// factors the columns took 366-434 us), and two real rows per transform instead of
+// the even/odd split (rows and residual 209 and 299 us with it, then 153 and 245).
 #pragma once
 
 #include "gbk_batched.cuh"
